@@ -14,6 +14,8 @@
 // representative once, reads the key's row count (the output size is an
 // exclusive scan of those counts) and copies the key's rows out: the probe
 // compares keys once per probe row, not once per build row of its key.
+// Fixed-width keys that pack into one 64-bit word take gbx_join_packed.cu
+// instead; this path serves STRING, STRUCT and wider keys, and empty sides.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,6 +24,7 @@
 
 #include "../../include/gbx.h"
 #include "gbx_host.hpp"
+#include "gbx_join.hpp"
 #include "gbx_rep.cuh"
 #include "gbx_scan.hpp"
 
@@ -332,6 +335,10 @@ int gbx_hash_join(const gbx_table_view* left, const gbx_table_view* right, int32
     const gbx_table_view* probe = swap ? right : left;
     const int64_t nb = build->columns[0].size;
     const int64_t np = probe->columns[0].size;
+    // keys of one packed word carry the key in the slot (gbx_join_packed.cu)
+    if (packed_join(build, probe, compare_nulls, join_kind, a, swap ? *right_indices : *left_indices,
+                    swap ? *left_indices : *right_indices))
+      return;
     const std::vector<gbx_column_view> bcols(build->columns, build->columns + build->num_columns);
     const std::vector<gbx_column_view> pcols(probe->columns, probe->columns + probe->num_columns);
     KeyTree tb = key_tree(bcols, GBX_NULL_INCLUDE);

@@ -1,0 +1,56 @@
+"""Joins whose key packs into one 64-bit word (gbx_join_packed.cu) against the
+join oracle: unique and repeated build keys, row counts around the 2,048-row
+probe tile, the all-ones key (the table's empty word), several key layouts,
+nulls and sliced columns.  Pairs are compared bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cudf_b200 import Table
+from cudf_b200 import join as J
+from cudf_b200._abi import JoinKind, NullEquality
+from oracle.oracle import HostCol
+from tests import gbx_testing as T
+from tests.test_gpu_join import KINDS, _check
+
+pytestmark = pytest.mark.gpu
+
+
+def _keys(layout, idx, rng):
+    """Key columns of the key numbers `idx`; number 0 is all ones where the layout allows it."""
+    if layout == "int64":
+        return [HostCol((idx.astype(np.int64) * 982_451_653) - 1)]
+    if layout == "int32":
+        return [HostCol(idx.astype(np.int32) - 1)]
+    if layout == "int32_int16_nulls":
+        valid = (idx % 7) != 3  # a null key column, the same for equal numbers
+        return [HostCol(idx.astype(np.int32) * 77), HostCol((idx % 1000).astype(np.int16), valid)]
+    v = (idx - 5).astype(np.float64) * 0.5
+    v[idx == 5] = np.where(rng.random(int((idx == 5).sum())) < 0.5, -0.0, 0.0)
+    v[idx == 9] = np.nan
+    return [HostCol(v)]
+
+
+@pytest.mark.parametrize("layout", ["int64", "int32", "int32_int16_nulls", "float64"])
+@pytest.mark.parametrize("repeated", [False, True], ids=["unique", "repeated"])
+@pytest.mark.parametrize("nl,nr", [(1, 1), (2047, 60), (2048, 700), (2049, 3000), (6145, 1500)])
+def test_packed_join_matches_oracle(layout, repeated, nl, nr):
+    rng = np.random.default_rng(nl * 7 + nr)
+    right = rng.integers(0, max(1, nr // 3), nr) if repeated else rng.permutation(nr)
+    left = rng.integers(0, max(2, nr + nr // 4), nl)
+    left[0] = 0
+    for kind in KINDS:
+        for nulls in (NullEquality.EQUAL, NullEquality.UNEQUAL):
+            _check(_keys(layout, left, rng), _keys(layout, right, rng), nulls, kind)
+
+
+def test_packed_join_of_sliced_columns():
+    rng = np.random.default_rng(5)
+    a, b = rng.integers(0, 300, 5000), rng.permutation(400)
+    left = Table([T.device_column(HostCol(a.astype(np.int64))).slice(13, 4111)])
+    right = Table([T.device_column(HostCol(b.astype(np.int64))).slice(7, 390)])
+    li, ri = (c.to_numpy()[0] for c in J.inner_join(left, right))
+    where = {int(k): i for i, k in enumerate(b[7:390])}
+    want = [(i, where[int(k)]) for i, k in enumerate(a[13:4111]) if int(k) in where]
+    assert sorted(zip(li.tolist(), ri.tolist())) == want
