@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "gbx_batch.hpp"
+#include "gbx_rows.cuh"
 #include "gbx_scan.hpp"
 #include "gbx_warpcore.cuh"
 
@@ -77,11 +78,120 @@ struct LoadedRow {
 
 // --------------------------------------------------------- per-item modes
 
+// Rows a thread of item_shared takes at a time.
+constexpr int kSharedPer = 4;
+
+// Channel c's values and validity (bit q of the result) of an instance's rows
+// r0 + q * step.
+__device__ __forceinline__ uint32_t inst_rows(const Plan& plan, const InstCols& ic, int c, int64_t r0, int step,
+                                              uint32_t rows, uint64_t (&v)[kSharedPer], int32_t* status)
+{
+  const InstChan& ch = ic.chan[c];
+  if (ch.dict_data == nullptr) {
+    load_rows<kSharedPer>(pt_width(plan.chan[c].ptype), ch.data, r0 + ch.offset, step, rows, v);
+    return valid_rows<kSharedPer>(ch.mask, r0 + ch.offset, step, rows);
+  }
+  const BatchSource src{&plan, &ic};
+  uint32_t ok = 0;
+#pragma unroll
+  for (int q = 0; q < kSharedPer; ++q) {
+    v[q] = 0;
+    if (((rows >> q) & 1u) && src.value(c, r0 + static_cast<int64_t>(q) * step, v[q], status)) ok |= 1u << q;
+  }
+  __syncwarp();
+  return ok;
+}
+
+// Folds one channel's values into their rows' slots with shared atomics, one
+// accumulator at a time over the thread's rows.  An extreme is only written
+// when it beats the one read (a slot's extremes settle early).  The warp
+// meets again after each floating add (a compare-and-swap loop).
+template <int PT>
+__device__ __forceinline__ void apply_rows(const Channel& ch, const Level<Shared>& L, const uint32_t (&slot)[kSharedPer],
+                                           uint32_t rows, const uint64_t (&v)[kSharedPer], int32_t* status)
+{
+  constexpr bool kFloat = PT == P_F32 || PT == P_F64;
+  constexpr bool kM64   = PT == P_I64 || PT == P_U64 || PT == P_F64;
+#define GBX_ROWS(...)                                          \
+  _Pragma("unroll") for (int q = 0; q < kSharedPer; ++q) {     \
+    if ((rows >> q) & 1u) { __VA_ARGS__ }                      \
+  }
+#define GBX_ROWS_MEET(...)                                     \
+  _Pragma("unroll") for (int q = 0; q < kSharedPer; ++q) {     \
+    if ((rows >> q) & 1u) { __VA_ARGS__ }                      \
+    __syncwarp();                                              \
+  }
+  if (ch.a_cnt >= 0) GBX_ROWS(Shared::add_u32(L.acc(ch.a_cnt) + slot[q] * 4, 1u);)
+  if (ch.a_min >= 0) {
+    if constexpr (kM64)
+      GBX_ROWS(const uint64_t e = enc_minmax(v[q], PT, true); const uint32_t a = L.acc(ch.a_min) + slot[q] * 8;
+               if (e < Shared::ld_u64(a)) Shared::min_u64(a, e);)
+    else
+      GBX_ROWS(const uint32_t e = static_cast<uint32_t>(enc_minmax(v[q], PT, true));
+               const uint32_t a = L.acc(ch.a_min) + slot[q] * 4; if (e < Shared::ld_u32(a)) Shared::min_u32(a, e);)
+  }
+  if (ch.a_max >= 0) {
+    if constexpr (kM64)
+      GBX_ROWS(const uint64_t e = enc_minmax(v[q], PT, false); const uint32_t a = L.acc(ch.a_max) + slot[q] * 8;
+               if (e > Shared::ld_u64(a)) Shared::max_u64(a, e);)
+    else
+      GBX_ROWS(const uint32_t e = static_cast<uint32_t>(enc_minmax(v[q], PT, false));
+               const uint32_t a = L.acc(ch.a_max) + slot[q] * 4; if (e > Shared::ld_u32(a)) Shared::max_u32(a, e);)
+  }
+  if constexpr (kFloat) {
+    if (ch.a_sum >= 0) GBX_ROWS_MEET(Shared::add_f64(L.acc(ch.a_sum) + slot[q] * 8, as_f64(v[q], PT));)
+    if (ch.a_sq >= 0)
+      GBX_ROWS_MEET(const double x = as_f64(v[q], PT); Shared::add_f64(L.acc(ch.a_sq) + slot[q] * 8, x * x);)
+    if (ch.a_prod >= 0) GBX_ROWS_MEET(mul_cas_f64<Shared>(L.acc(ch.a_prod) + slot[q] * 8, as_f64(v[q], PT), status);)
+  } else {
+    if (ch.a_sum >= 0)
+      GBX_ROWS(Shared::add_u64(L.acc(ch.a_sum) + slot[q] * 8, static_cast<uint64_t>(as_i64(v[q], PT)));)
+    if (ch.a_sq >= 0)
+      GBX_ROWS(const uint64_t x = static_cast<uint64_t>(as_i64(v[q], PT));
+               Shared::add_u64(L.acc(ch.a_sq) + slot[q] * 8, x * x);)
+    if (ch.a_prod >= 0) GBX_ROWS_MEET(mul_cas_i64<Shared>(L.acc(ch.a_prod) + slot[q] * 8, as_i64(v[q], PT), status);)
+  }
+  if (ch.a_k >= 0) {
+    GBX_ROWS_MEET(const double x = as_f64(v[q], PT); const double K = get_shift<Shared>(L.acc(ch.a_k) + slot[q] * 8, x);
+                  const double d = x - K; Shared::add_f64(L.acc(ch.a_s2) + slot[q] * 8, d * d);
+                  if (kFloat) Shared::add_f64(L.acc(ch.a_s1) + slot[q] * 8, d);)
+  }
+#undef GBX_ROWS
+#undef GBX_ROWS_MEET
+}
+
+// The bits q of `rows`: rows r0 + q * step straight into the global table.
+template <int NW>
+__device__ __noinline__ void spill_rows(const Plan& plan, const BatchInst& I, int64_t r0, int step, uint32_t rows,
+                                        uint32_t max_probes)
+{
+  const BatchSource src{&plan, &I.cols};
+  const Level<Global> G{&I.t};
+  for (int q = 0; q < kSharedPer; ++q) {
+    if ((rows >> q) & 1u) {
+      const int64_t r = r0 + static_cast<int64_t>(q) * step;
+      uint64_t k[NW];
+      src.key<NW>(r, k);
+      const int64_t g = global_slot<NW>(I.t, k, max_probes);
+      if (g >= 0) accumulate_row_from<Global>(plan, src, G, g, r, I.t.status);
+    }
+    __syncwarp();
+  }
+}
+
 // CTA-shared table with shared-memory atomics; rows whose key finds no room
 // go to the global table; the table is merged into the global one at the end.
-template <int NW, int NCH, int BLOCK>
+//
+// Bound by the shared-memory atomics and the instructions around them, so a
+// thread takes kSharedPer rows through each step together and every 64-bit
+// integer sum is a pair of native 32-bit adds (Shared::add_u64).  Measured on
+// B200, 4,096 instances (594M rows; SUM, COUNT, MAX of int64 by an int32 key):
+// one row a thread at a time with 64-bit compare-and-swap adds 22.5 ms, this
+// 15.5 ms under the same plan (per class of group counts: 10 to 500 groups 27-31
+// -> 87-127 G rows/s).
+template <int NW, int BLOCK>
 __device__ __forceinline__ void item_shared(const Plan& plan, const BatchInst& I, unsigned char* smem,
-                                            uint32_t& s_special, int64_t begin, int64_t end)
+                                            int64_t begin, int64_t end)
 {
   const SmemLayout& sl = I.sl;
   const uint32_t S     = sl.slots;
@@ -100,44 +210,47 @@ __device__ __forceinline__ void item_shared(const Plan& plan, const BatchInst& I
   }
   __syncthreads();
 
-  const BatchSource src{&plan, &I.cols};
   const Level<Shared> L{base, &sl};
   const Level<Global> G{&I.t};
   const uint32_t keys        = base + sl.keys_off;
   const uint32_t smem_probes = S < 32 ? S : 32;
   const uint32_t max_probes  = probe_limit(I.t.cap);
-  // the next row's key and values load while this row is applied
-  int64_t r = begin + threadIdx.x;
-  uint64_t k[NW];
-  bool act = r < end && src.key<NW>(r, k);
-  RowVals<NCH> v;
-  load_row_values(plan, src, act, r, v, I.t.status);
-  for (; r < end; r += BLOCK) {
-    const int64_t rn = r + BLOCK;
-    uint64_t kn[NW];
-    const bool actn = rn < end && src.key<NW>(rn, kn);
-    RowVals<NCH> vn;
-    load_row_values(plan, src, actn, rn, vn, I.t.status);
-    if (act) {
-      int64_t s;
-      if (key_is_empty<NW>(k)) {
-        s = S;
-        if (s_special == 0) s_special = 1;
-      } else {
-        s = find_or_insert<Shared, NW>(keys, S - 1, k, hash_key<NW>(k), smem_probes);
-      }
-      const LoadedRow<NCH> lr{&v};
-      if (s >= 0) {
-        accumulate_row_from<Shared>(plan, lr, L, s, r, I.t.status);
-      } else {
-        const int64_t g = global_slot<NW>(I.t, k, max_probes);
-        if (g >= 0) accumulate_row_from<Global>(plan, lr, G, g, r, I.t.status);
-      }
-    }
-    act = actn;
+  // kSharedPer rows a thread at a time (the whole warp stays in the loop)
+  for (int64_t r0 = begin + threadIdx.x; r0 - threadIdx.x < end; r0 += kSharedPer * BLOCK) {
+    uint32_t kept = 0;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) k[w] = kn[w];
-    v = vn;
+    for (int q = 0; q < kSharedPer; ++q) kept |= r0 + q * BLOCK < end ? 1u << q : 0u;
+    uint64_t k[kSharedPer][NW];
+    kept = pack_rows<kSharedPer, NW>(plan.key, InstKeyBufs{&I.cols}, r0, BLOCK, kept, k);
+    uint64_t v[kSharedPer];
+    uint32_t ok = 0;
+    if (plan.nchan > 0) ok = inst_rows(plan, I.cols, 0, r0, BLOCK, kept, v, I.t.status);
+    uint32_t slot[kSharedPer];
+    const uint32_t found = find_slots<kSharedPer, NW>(skeys, keys, S - 1, kept, k, smem_probes, slot);
+    // rows without a slot go to the global table
+    if (__any_sync(kFull, found != kept)) spill_rows<NW>(plan, I, r0, BLOCK, kept & ~found, max_probes);
+#pragma unroll
+    for (int q = 0; q < kSharedPer; ++q)
+      if ((found >> q) & 1u) Shared::add_u32(L.rows() + slot[q] * 4, 1u);
+    for (int c = 0; c < plan.nchan; ++c) {
+      const Channel& ch = plan.chan[c];
+      if (c > 0) ok = inst_rows(plan, I.cols, c, r0, BLOCK, kept, v, I.t.status);
+#define GBX_APPLY(P) apply_rows<P>(ch, L, slot, ok & found, v, I.t.status); break;
+      switch (ch.ptype) {
+        case P_I8: GBX_APPLY(P_I8)
+        case P_I16: GBX_APPLY(P_I16)
+        case P_I32: GBX_APPLY(P_I32)
+        case P_I64: GBX_APPLY(P_I64)
+        case P_U8: GBX_APPLY(P_U8)
+        case P_U16: GBX_APPLY(P_U16)
+        case P_U32: GBX_APPLY(P_U32)
+        case P_U64: GBX_APPLY(P_U64)
+        case P_F32: GBX_APPLY(P_F32)
+        case P_F64: GBX_APPLY(P_F64)
+        default: GBX_APPLY(P_BOOL)
+      }
+#undef GBX_APPLY
+    }
   }
   __syncthreads();
 
@@ -145,8 +258,7 @@ __device__ __forceinline__ void item_shared(const Plan& plan, const BatchInst& I
     uint64_t k[NW];
 #pragma unroll
     for (int w = 0; w < NW; ++w) k[w] = skeys[s * NW + w];
-    const bool occupied = (s < S) ? !key_is_empty<NW>(k) : (s_special != 0);
-    if (!occupied) continue;
+    if (srows[s] == 0) continue;
     const int64_t g = global_slot<NW>(I.t, k, max_probes);
     if (g >= 0) merge_slot<Shared>(plan, L, s, G, g, I.t.status);
   }
@@ -247,7 +359,7 @@ __device__ __forceinline__ void item_global(const Plan& plan, const BatchInst& I
 // ---------------------------------------------------------------- kernels
 
 template <int NW, int NCH, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_batch_agg(const __grid_constant__ Plan plan,
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_batch_agg(const __grid_constant__ Plan plan,
                                                                   const BatchInst* __restrict__ insts,
                                                                   const BatchItem* __restrict__ items,
                                                                   uint32_t nitems,
@@ -256,7 +368,6 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_batch_agg(const __grid_c
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ BatchInst s_inst;
   __shared__ uint32_t s_item;
-  __shared__ uint32_t s_special;
   static_assert(sizeof(BatchInst) % 16 == 0, "BatchInst is copied as 16-byte vectors");
 
   for (;;) {
@@ -270,10 +381,9 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_batch_agg(const __grid_c
       uint4* dst       = reinterpret_cast<uint4*>(&s_inst);
       for (int i = threadIdx.x; i < static_cast<int>(sizeof(BatchInst) / 16); i += BLOCK) dst[i] = __ldg(src + i);
     }
-    if (threadIdx.x == 0) s_special = 0;
     __syncthreads();
     switch (s_inst.mode) {
-      case BM_SHARED: item_shared<NW, NCH, BLOCK>(plan, s_inst, smem, s_special, item.begin, item.end); break;
+      case BM_SHARED: item_shared<NW, BLOCK>(plan, s_inst, smem, item.begin, item.end); break;
       case BM_WARP: item_warp<NW, NCH, BLOCK>(plan, s_inst, smem, item.begin, item.end); break;
       default: item_global<NW, NCH, BLOCK>(plan, s_inst, item.begin, item.end); break;
     }

