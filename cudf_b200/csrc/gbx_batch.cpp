@@ -30,20 +30,24 @@ using namespace gbx;
 namespace gbx {
 namespace {
 
-// Dynamic shared memory per CTA for the two block shapes the tuner picks
-// from: 256 threads with two CTAs per SM, or 512 threads with one.
+// Dynamic shared memory per CTA.  The tuner picks from 512 threads with one or
+// two CTAs an SM and 1,024 with one: a table beyond half an SM's shared memory
+// leaves room for one CTA, which then needs all the threads (measured on the
+// class of 1,024-2,047 groups: 512 threads 54 G rows/s, 1,024 90 G).  256
+// threads, at most 100 KB each, measured below both in every class; a caller
+// may still ask for them.
 constexpr size_t kSmemBudget256  = 100 * 1024;
-constexpr size_t kSmemBudget512  = kBatchMaxDynamicSmem;
+constexpr size_t kSmemBudgetBig  = kBatchMaxDynamicSmem;
 constexpr int kSamplePerInstance = 2048;
 constexpr int kMinTileLog2       = 12;
 constexpr int kMaxTileLog2       = 20;
 
-size_t smem_budget(int block) { return block == 512 ? kSmemBudget512 : kSmemBudget256; }
+size_t smem_budget(int block) { return block >= 512 ? kSmemBudgetBig : kSmemBudget256; }
 
 // One tuned choice for a class of instances under one block shape.
 struct Choice {
   int32_t mode      = BM_GLOBAL;
-  int32_t smul      = 0;   // shared table slots = base_slots(class) << smul
+  int32_t smul      = 0;   // shared table slots = base_slots(class) * 2^smul, smul -1 to 2
   int32_t tile_log2 = 16;  // rows per work item
   double rate       = 0;   // measured rows/s of the class (0: not measured)
 };
@@ -62,6 +66,15 @@ uint32_t base_slots(int cls)
 {
   uint64_t s = next_pow2(static_cast<uint64_t>(std::ceil(std::ldexp(1.0, cls + 1) * 1.25)));
   return static_cast<uint32_t>(std::max<uint64_t>(s, 32));
+}
+
+// Slots under a choice.  smul -1 loads the table up to 1.25 times its slots
+// at the class's upper end (the rows of the last groups then go to the global
+// table): it still wins for classes whose full table does not fit.
+uint32_t choice_slots(int cls, int smul)
+{
+  const uint32_t s = base_slots(cls);
+  return smul < 0 ? std::max<uint32_t>(s >> 1, 32) : s << smul;
 }
 
 // ---------------------------------------------------------- tuning table
@@ -91,8 +104,8 @@ std::map<TuneKey, Choice> read_tune_file(const char* path)
     TuneKey k;
     Choice c;
     if (!(is >> k.device >> k.sig >> k.block >> k.cls >> c.mode >> c.smul >> c.tile_log2 >> c.rate)) continue;
-    if (c.mode < BM_SHARED || c.mode > BM_GLOBAL || c.smul < 0 || c.smul > 2 || c.tile_log2 < kMinTileLog2 ||
-        c.tile_log2 > kMaxTileLog2 || (k.block != 256 && k.block != 512))
+    if (c.mode < BM_SHARED || c.mode > BM_GLOBAL || c.smul < -1 || c.smul > 2 || c.tile_log2 < kMinTileLog2 ||
+        c.tile_log2 > kMaxTileLog2 || (k.block != 256 && k.block != 512 && k.block != 1024))
       continue;
     m[k] = c;
   }
@@ -396,7 +409,7 @@ void apply_choice(gbx_batch& b, gbx_batch::Inst& I, const Choice& c, int64_t til
   I.mode = c.mode;
   I.S    = 0;
   if (c.mode == BM_SHARED || c.mode == BM_WARP) {
-    uint32_t S        = base_slots(I.cls) << c.smul;
+    uint32_t S        = choice_slots(I.cls, c.smul);
     const size_t need = (c.mode == BM_WARP ? b.block / 32 : 1) * static_cast<size_t>(make_smem_layout(b.schema, S).total);
     if (need > smem_budget(b.block)) I.mode = BM_GLOBAL;
     else I.S = S;
@@ -698,7 +711,7 @@ void plan_batch(gbx_batch& b, const gbx_batch_options& o)
     table = read_tune_file(o.tune_file);
   }
   std::vector<std::pair<TuneKey, Choice>> fresh;
-  const std::vector<int> blocks = o.block_threads ? std::vector<int>{o.block_threads} : std::vector<int>{256, 512};
+  const std::vector<int> blocks = o.block_threads ? std::vector<int>{o.block_threads} : std::vector<int>{512, 1024};
   std::map<int, std::map<int, Choice>> chosen;  // block -> class -> choice
   int measured = 0, cached = 0;
   for (int blk : blocks) {
@@ -709,19 +722,21 @@ void plan_batch(gbx_batch& b, const gbx_batch_options& o)
       auto it         = table.find(key);
       const bool have = it != table.end() && it->second.rate > 0;
       if (o.tune == GBX_TUNE_ALL || (o.tune == GBX_TUNE_MISSING && !have)) {
-        // representatives: the class's largest instances, up to ~16M rows
+        // representatives: the class's largest instances, up to ~64M rows
+        // (fewer leave SMs idle under the larger tiles, which then lose
+        // although a batch has items for every SM)
         std::vector<int> members = kv.second;
         std::stable_sort(members.begin(), members.end(), [&](int x, int y) { return b.inst[x].n > b.inst[y].n; });
         std::vector<int> subset;
         int64_t rows = 0;
         for (int i : members) {
-          if (subset.size() >= 64 || rows >= (int64_t(16) << 20)) break;
+          if (subset.size() >= 256 || rows >= (int64_t(64) << 20)) break;
           subset.push_back(i);
           rows += b.inst[i].n;
         }
         std::vector<Choice> cand;
         for (int tl : {15, 17}) {
-          for (int smul = 0; smul <= 1; ++smul) {
+          for (int smul = -1; smul <= 1; ++smul) {
             Choice c;
             c.mode = BM_SHARED, c.smul = smul, c.tile_log2 = tl;
             cand.push_back(c);

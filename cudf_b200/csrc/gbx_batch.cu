@@ -591,6 +591,10 @@ cudaError_t dispatch(const Plan& p, int block, Args&&... args)
 {
   const bool nw1 = p.key.nwords == 1;
   const bool c2  = p.nchan <= 2;
+  if (block == 1024) {
+    if (nw1) return c2 ? F<1, 2, 1024>::run(args...) : F<1, kMaxChannels, 1024>::run(args...);
+    return c2 ? F<2, 2, 1024>::run(args...) : F<2, kMaxChannels, 1024>::run(args...);
+  }
   if (block == 512) {
     if (nw1) return c2 ? F<1, 2, 512>::run(args...) : F<1, kMaxChannels, 512>::run(args...);
     return c2 ? F<2, 2, 512>::run(args...) : F<2, kMaxChannels, 512>::run(args...);

@@ -25,8 +25,9 @@ namespace gbx {
 enum BatchMode : int32_t { BM_SHARED = 1, BM_WARP = 2, BM_GLOBAL = 3 };
 
 // Dynamic shared memory limit set once on the aggregation kernel, so that a
-// graph captured with any size up to it stays launchable.
-constexpr size_t kBatchMaxDynamicSmem = 200 * 1024;
+// graph captured with any size up to it stays launchable (the 227 KB a block
+// may use, less the kernel's static shared memory).
+constexpr size_t kBatchMaxDynamicSmem = 225 * 1024;
 
 struct InstKeyCol {
   const void* data;
@@ -77,7 +78,7 @@ cudaError_t launch_batch_sample(const Plan& schema, const BatchInst* insts, int 
 cudaError_t launch_batch_init(const Plan& schema, const BatchInst* insts, int ninst, cudaStream_t st);
 
 // The persistent aggregation kernel over `nitems` items (claimed through
-// *counter, which must be zero).  `block` is 256 or 512; `grid` CTAs with
+// *counter, which must be zero).  `block` is 256, 512 or 1,024; `grid` CTAs with
 // `smem` bytes of dynamic shared memory each (batch_agg_max_grid first).
 cudaError_t launch_batch_agg(const Plan& schema, const BatchInst* insts, const BatchItem* items, uint32_t nitems,
                              uint32_t* counter, int block, int grid, size_t smem, cudaStream_t st);
