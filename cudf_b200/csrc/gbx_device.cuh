@@ -439,6 +439,14 @@ __device__ __forceinline__ int64_t find_or_insert(typename Space::addr_t keys,
     } else {
       uint64_t c0 = Space::ld_u64(a);
       uint64_t c1 = Space::ld_u64(a + 8);
+      // The two loads may straddle the slot's insertion: a key with an
+      // all-ones word then matches that word still empty beside the other
+      // word of a different key.  The other word was seen written, so a
+      // second look reads the slot's final key.
+      if (c0 == k[0] && c1 == k[1] && (c0 == kEmptyWord || c1 == kEmptyWord)) {
+        c0 = Space::ld_u64(a);
+        c1 = Space::ld_u64(a + 8);
+      }
       if (c0 == k[0] && c1 == k[1]) return static_cast<int64_t>(s);
       if (c0 == kEmptyWord || c1 == kEmptyWord) {
         // empty or being written: the 128-bit CAS decides
