@@ -990,7 +990,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     for (int bb : {8, 16}) {
       const double groups = est / (2.0 * call.dev.num_sms) + est / static_cast<double>(1u << bb);
       const auto Sb = static_cast<uint32_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * groups, 64.0))));
-      if (Sb <= 1024 && tiled_fits(make_smem_layout(plan, Sb), plan.nchan)) {
+      if (Sb <= 1024 && tiled_fits(make_smem_layout(plan, Sb), plan, /*two_per_sm=*/true)) {
         bucket_bits  = bb;
         bucket_slots = Sb;
         break;
@@ -1002,7 +1002,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       // that fits (rows of groups beyond it go to the global table directly)
       bucket_bits = 16;
       for (uint32_t Sb = 1024; Sb >= 64 && bucket_slots == 0; Sb >>= 1)
-        if (tiled_fits(make_smem_layout(plan, Sb), plan.nchan)) bucket_slots = Sb;
+        if (tiled_fits(make_smem_layout(plan, Sb), plan)) bucket_slots = Sb;
       if (bucket_slots == 0) strategy = GBX_STRATEGY_GLOBAL;
     }
     // Skewed keys: when the keys sampled 4 or more times hold most sampled
@@ -1404,7 +1404,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
           // a short probe: a hot key was inserted early and sits near its home
           // slot; a rare key that misses goes to the global table
           GBX_CUDA(launch_agg_stream(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 8), max_probes, s));
-        } else if (tiled_fits(sl, plan.nchan) && !arg_kinds) {
+        } else if (tiled_fits(sl, plan) && !arg_kinds) {
           // few groups: tiles grouped in shared memory before the table is touched
           GBX_CUDA(launch_agg_tiled(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 32), max_probes, s));
         } else {

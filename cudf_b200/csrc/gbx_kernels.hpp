@@ -53,10 +53,11 @@ cudaError_t launch_agg_global(const Plan& p, const TableRef& t, int64_t n, uint3
                               cudaStream_t st);
 cudaError_t launch_agg_privatized(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int block,
                                   int grid, uint32_t smem_probes, uint32_t max_probes, cudaStream_t st);
-// Per-CTA tables fed by tile-local grouping (gbx_tiled.cu), for tables where
-// tiled_fits() (at most 1,024 slots, table and a tile's staged values within
-// half an SM's shared memory).
-bool tiled_fits(const SmemLayout& sl, int nchan);
+// Per-CTA tables fed by tile-local grouping (gbx_tiled.cu; ARGMIN / ARGMAX are
+// not computed), for tables where tiled_fits() (at most 4,096 slots, table
+// and a tile's staged values within an SM's shared memory, or within half of
+// it with two_per_sm).
+bool tiled_fits(const SmemLayout& sl, const Plan& p, bool two_per_sm = false);
 // Streamed tiles grouped in shared memory (gbx_stream.cu): one packed key
 // word, no ARGMIN/ARGMAX, a table of at most 4,096 slots.
 bool stream_fits(const Plan& p, const SmemLayout& sl);

@@ -162,6 +162,8 @@ __device__ __forceinline__ uint32_t find_slots(uint64_t* skeys, uint32_t keys_sa
     bool hit = true;
 #pragma unroll
     for (int w = 0; w < NW; ++w) hit = hit && skeys[slot[q] * NW + w] == k[q][w];
+    // a key with an all-ones word may match a slot being written: find_or_insert settles it
+    if constexpr (NW == 2) hit = hit && k[q][0] != kEmptyWord && k[q][1] != kEmptyWord;
     // an all-ones key also matches an empty slot: it takes the reserved one
     if (key_is_empty<NW>(k[q])) {
       slot[q] = mask + 1;

@@ -1,30 +1,48 @@
-// gbx_tiled.cu -- low-cardinality aggregation by grouping each tile of rows
-// before touching the table.
+// gbx_tiled.cu -- aggregation by grouping each tile of rows in shared memory
+// before touching the CTA's table.
 //
-// With few groups (up to ~500) every CTA holds the whole group table in shared
-// memory.  Applying each row to it costs ~13 shared-memory atomics per row for
-// the 100M-row workload's 12 accumulators, and the 64-bit ones run as
-// compare-and-swap loops that conflict when many lanes hit the same few slots:
-// the per-row atomic path measured 35.7 warp-instructions per row on B200.
-// Here a CTA instead takes up to 4,096 rows at a time and
-//   1. loads the tile's keys and, per channel, its values and validity into
-//      shared memory (coalesced, every load of a batch in flight together),
-//      then finds each row's slot in its table and takes the next rank of that
-//      slot with one 32-bit shared atomic;
-//   2. scans the slot counts and lists the tile's rows group by group;
-//   3. folds each group's rows in one thread's registers (ChanAcc), reading the
-//      staged values, then merges that into the group's slot with plain
-//      read-modify-writes -- the thread owns the slot for the step, so no
-//      atomics are needed.
-// A group with r rows in the tile updates its slot once instead of r times.
-// Rows whose key finds no room in the table go to the global table directly,
-// and every CTA merges its table into the global one at the end, as the
-// per-CTA privatised kernel does (the reference's shared-memory aggregation,
-// hash/groupby.cu:424-504, restated with tile-local grouping).
-#include <cub/block/block_scan.cuh>
-
+// Applying rows one by one to a shared table costs ~13 shared-memory atomics
+// a row for the 100M-row workload's 12 accumulators, and the 64-bit ones run
+// as compare-and-swap loops that conflict when many lanes hit the same few
+// slots (35.7 warp-instructions a row).  Here a CTA takes up to 8 rows a
+// thread at a time and
+//   1. packs the tile's keys column by column (one uniform branch on a key
+//      column's width serves all of a thread's rows), finds each row's slot
+//      in its table and takes the next rank of that slot with one 32-bit
+//      shared atomic; rows whose key finds no slot are listed and sent to the
+//      global table by the whole CTA together;
+//   2. scans the slots' (rows, chunks of at most kChunk rows) in one pass;
+//   3. stores each channel's values, at their own width, at their row's
+//      position, so that the tile lies in shared memory group by group (the
+//      first channel's loads are in flight across the scan);
+//   4. folds one chunk per thread in registers, four consecutive values at a
+//      time, and merges it into the group's slot with shared atomics; a warp
+//      whose 32 chunks are all of one group adds them with shuffles first.
+// After its last tile the CTA merges its table into the global one, as the
+// reference's shared-memory aggregation does (hash/groupby.cu:424-504).
+//
+// Issue-bound (57% of issue slots, 16.6 warp-instructions a row): the work per
+// row is a hash, a probe, a rank, one staged store and load per channel and
+// the fold itself.  The warp meets again after every probe loop and every
+// compare-and-swap loop; where it did not, the lanes ran all that followed
+// apart (11 active lanes an instruction, 33 warp-instructions a row).  The four-wide folds keep the
+// tests for the accumulators a plan uses, and the loop control, at a quarter
+// of an instruction a row.  Two CTAs of 512 threads an SM where the table and
+// the tile fit half its shared memory, so that one folds while the other
+// waits for its loads; one of 1,024 threads for larger tables.
+//
+// The caller's rows are dealt to the CTAs tile by tile; the bucket-ordered
+// copies of the radix partitioning (PART) in one contiguous run per CTA.
+//
+// Measured on B200, 100M rows, 12 accumulators, against the kernel this
+// replaces (per-slot folds of values read through a permutation, the warp
+// apart after each probe): 100 groups 3,586 -> 2,528 us, bucket-ordered copies
+// of 1e4 groups 4,257 -> 2,608 us; 10M rows, 1,000 groups, five aggregations
+// of one double column, 384 us with per-row shared atomics -> 254 us.
 #include <algorithm>
+#include <type_traits>
 
+#include "gbx_rows.cuh"
 #include "gbx_warpcore.cuh"
 
 namespace gbx {
@@ -33,409 +51,669 @@ using namespace dev;
 
 namespace {
 
-constexpr int kTiledBlock    = 512;
-constexpr int kTiledPer      = 8;  // at most this many rows per thread per tile
-constexpr int kTiledMaxRows  = kTiledBlock * kTiledPer;
-constexpr int kTiledMaxSlots = 1024;
-constexpr int kScanPer       = (kTiledMaxSlots + 1 + kTiledBlock - 1) / kTiledBlock;
+constexpr int kPer           = 8;  // rows per thread and tile at most
+constexpr int kBatch         = 4;  // of which so many are in flight together
+constexpr int kChunk         = 16; // rows of one group folded by one thread
+constexpr int kMaxSlots      = 4096;
 constexpr uint32_t kNoRec    = 0xffffffffu;
-constexpr int kChunk         = 16;  // rows of one group folded by one thread
-// chunks of one tile: sum over groups of ceil(rows / kChunk)
-constexpr int kMaxChunks = kTiledMaxRows / kChunk + kTiledMaxSlots + 1;
-// dynamic shared memory per CTA so that two CTAs fit an SM (228 KB, less
-// 1 KB reserved and ~2 KB of static shared memory per CTA)
-constexpr size_t kTiledSmemBudget = 110 * 1024;
+// dynamic shared memory so that two CTAs of 512 threads fit an SM (228 KB,
+// less 1 KB reserved and the static shared memory per CTA), or one of 1,024
+constexpr size_t kSmemTwo = 112 * 1024;
+constexpr size_t kSmemOne = 225 * 1024;
 
-// Folds `len` staged rows of one group (tile-local indices rows[0..len)) of a
-// channel of physical type PT into A.
-template <int PT>
-__device__ __forceinline__ void fold_chunk(const Channel& ch, const uint64_t* cv, const uint8_t* cvv,
-                                           const uint16_t* rows, uint32_t len, ChanAcc& A)
-{
-  const uint32_t roles = chan_roles(ch);
-  for (uint32_t j = 0; j < len; ++j) {
-    const uint32_t li = rows[j];
-    if (cvv[li]) chan_acc_add<PT>(ch, roles, A, cv[li]);
-  }
-}
-
-// Merges a chunk's accumulators into slot s of the CTA table with shared
-// atomics (several chunks of a group merge at once).  The slot's shift was
-// fixed before the chunks were folded, so A.s2 and A.s1 are relative to it.
-__device__ __forceinline__ void merge_partial(const Channel& ch, const ChanAcc& A, const Level<Shared>& L, uint32_t s,
-                                              int32_t* status)
-{
-  if (A.cnt == 0) return;
-  if (ch.a_cnt >= 0) Shared::add_u32(L.acc(ch.a_cnt) + s * 4, A.cnt);
-  const bool m64 = minmax_is64(ch.ptype);
-  if (ch.a_min >= 0) {
-    if (m64) Shared::min_u64(L.acc(ch.a_min) + s * 8, A.mn);
-    else Shared::min_u32(L.acc(ch.a_min) + s * 4, static_cast<uint32_t>(A.mn));
-  }
-  if (ch.a_max >= 0) {
-    if (m64) Shared::max_u64(L.acc(ch.a_max) + s * 8, A.mx);
-    else Shared::max_u32(L.acc(ch.a_max) + s * 4, static_cast<uint32_t>(A.mx));
-  }
-  if (ch.is_float) {
-    if (ch.a_sum >= 0) Shared::add_f64(L.acc(ch.a_sum) + s * 8, __longlong_as_double(static_cast<long long>(A.sum)));
-    if (ch.a_sq >= 0) Shared::add_f64(L.acc(ch.a_sq) + s * 8, __longlong_as_double(static_cast<long long>(A.sq)));
-    if (ch.a_prod >= 0)
-      mul_cas_f64<Shared>(L.acc(ch.a_prod) + s * 8, __longlong_as_double(static_cast<long long>(A.prod)), status);
-  } else {
-    if (ch.a_sum >= 0) Shared::add_u64(L.acc(ch.a_sum) + s * 8, A.sum);
-    if (ch.a_sq >= 0) Shared::add_u64(L.acc(ch.a_sq) + s * 8, A.sq);
-    if (ch.a_prod >= 0) mul_cas_i64<Shared>(L.acc(ch.a_prod) + s * 8, static_cast<int64_t>(A.prod), status);
-  }
-  if (ch.a_k >= 0) Shared::add_f64(L.acc(ch.a_s2) + s * 8, A.s2);
-  if (ch.a_s1 >= 0) Shared::add_f64(L.acc(ch.a_s1) + s * 8, A.s1);
-}
-
-// Byte offsets of the per-tile staging areas in dynamic shared memory, after
-// the table: slot counts, first positions and first chunks ((S + 1) u32
-// each), the slot of each chunk (u16), the tile's rows in group order (u16),
-// each channel's value bits (u64) and validity bytes for tile_rows rows.
+// Byte offsets of the per-tile areas in dynamic shared memory, after the
+// table: slot counts ((S + 1) u32), each slot's first position and chunk
+// ((S + 2) u32: chunk << 16 | position), each row's slot and rank (u32), the
+// slot of each chunk (u16), the rows that found no slot (u16), each channel's values at their width, and a
+// validity byte per row of a nullable channel.
 struct TiledLayout {
-  uint32_t cnt_off, off_off, coff_off, cslot_off, perm_off, vals_off, valid_off, total;
+  uint32_t cnt_off, oc_off, rec_off, cslot_off, spill_off, total;
+  uint32_t val_off[kMaxChannels];
+  uint32_t ok_off[kMaxChannels];  // 0: the channel has no nulls
   int tile_rows;
+  int block;
 };
 
-TiledLayout tiled_layout(const SmemLayout& sl, int nchan, int tile_rows)
+TiledLayout tiled_layout(const SmemLayout& sl, const Plan& p, int block, int tile_rows)
 {
   TiledLayout tl{};
+  tl.block     = block;
   tl.tile_rows = tile_rows;
-  uint32_t o   = sl.total;
+  uint32_t o   = (sl.total + 15) & ~15u;
   tl.cnt_off   = o;
   o += (sl.slots + 1) * 4;
-  tl.off_off = o;
-  o += (sl.slots + 1) * 4;
-  tl.coff_off = o;
-  o += (sl.slots + 1) * 4;
+  tl.oc_off = o;
+  o += (sl.slots + 2) * 4;
+  tl.rec_off = o;
+  o += tile_rows * 4;
   tl.cslot_off = o;
-  o += kMaxChunks * 2;
-  tl.perm_off = o;
+  o += (tile_rows / kChunk + sl.slots + 2) * 2;
+  tl.spill_off = o;
   o += tile_rows * 2;
-  o           = (o + 7) & ~7u;
-  tl.vals_off = o;
-  o += static_cast<uint32_t>(nchan) * tile_rows * 8;
-  tl.valid_off = o;
-  o += static_cast<uint32_t>(nchan) * tile_rows;
+  for (int c = 0; c < p.nchan; ++c) {
+    o             = (o + 15) & ~15u;
+    tl.val_off[c] = o;
+    o += tile_rows * pt_width(p.chan[c].ptype);
+    if (p.chan[c].a_cnt >= 0) {
+      tl.ok_off[c] = o;
+      o += tile_rows;
+    }
+  }
   tl.total = (o + 15) & ~15u;
   return tl;
 }
 
-// The largest tile (a multiple of the block, at most kTiledMaxRows) whose
-// staging fits kTiledSmemBudget; tile_rows 0 when none does.
-TiledLayout pick_tiled_layout(const SmemLayout& sl, int nchan)
+// The largest tile that fits: two CTAs an SM when at least half a full tile
+// does, else one; tile_rows 0 when none fits.
+TiledLayout pick_tiled_layout(const SmemLayout& sl, const Plan& p)
 {
-  for (int rows = kTiledMaxRows; rows >= kTiledBlock; rows -= kTiledBlock) {
-    const TiledLayout tl = tiled_layout(sl, nchan, rows);
-    if (tl.total <= kTiledSmemBudget) return tl;
+  for (int rows = 512 * kPer; rows >= 512 * (kPer / 2); rows -= 512) {
+    const TiledLayout tl = tiled_layout(sl, p, 512, rows);
+    if (tl.total <= kSmemTwo) return tl;
   }
-  TiledLayout none{};
-  return none;
+  for (int rows = 1024 * kPer; rows >= 1024; rows -= 1024) {
+    const TiledLayout tl = tiled_layout(sl, p, 1024, rows);
+    if (tl.total <= kSmemOne) return tl;
+  }
+  return TiledLayout{};
 }
 
-// PART: the rows are the bucket-ordered copies `pb` of the radix
-// partitioning (*n_part of them) and each CTA takes one contiguous run of
-// tiles, so that its table only sees the groups of the few buckets the run
-// covers; otherwise the caller's n rows, tiles dealt round-robin.
+// Channel c's value bits and validity (bit q of the result) of this thread's
+// rows r0 + q * step (a plain or copied column).
+template <bool PART>
+__device__ __forceinline__ uint32_t channel_rows(const Plan& plan, const PartBufs& pb, int c, int64_t r0, int step,
+                                                 uint32_t rows, uint64_t (&v)[kBatch])
+{
+  if constexpr (PART) {
+    const PartCol& pc = pb.col[c];
+    load_rows<kBatch>(pc.width, pc.vals, r0, step, rows, v);
+    uint32_t ok = rows;
+    if (pc.valid != nullptr) {
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q)
+        if (((rows >> q) & 1u) && __ldg(pc.valid + r0 + static_cast<int64_t>(q) * step) == 0) ok &= ~(1u << q);
+    }
+    return ok;
+  } else {
+    const Channel& ch = plan.chan[c];
+    load_rows<kBatch>(pt_width(ch.ptype), ch.data, r0 + ch.offset, step, rows, v);
+    return valid_rows<kBatch>(ch.mask, r0 + ch.offset, step, rows);
+  }
+}
+
+// The same through a dictionary, for the rows that found a slot only (an
+// excluded row's index is not looked at).
+__device__ __noinline__ uint32_t dict_rows(const Plan& plan, int c, int64_t r0, int step, uint32_t rows,
+                                           uint64_t (&v)[kBatch], int32_t* status)
+{
+  const RowSource src{&plan};
+  uint32_t ok = 0;
+  for (int q = 0; q < kBatch; ++q) {
+    v[q] = 0;
+    if (((rows >> q) & 1u) && src.value(c, r0 + static_cast<int64_t>(q) * step, v[q], status)) ok |= 1u << q;
+  }
+  return ok;
+}
+
+// ------------------------------------------------------------- the fold
+
+template <int PT>
+struct Staged {
+  using type = unsigned long long;
+};
+template <>
+struct Staged<P_I8> { using type = uint8_t; };
+template <>
+struct Staged<P_U8> { using type = uint8_t; };
+template <>
+struct Staged<P_BOOL> { using type = uint8_t; };
+template <>
+struct Staged<P_I16> { using type = uint16_t; };
+template <>
+struct Staged<P_U16> { using type = uint16_t; };
+template <>
+struct Staged<P_I32> { using type = uint32_t; };
+template <>
+struct Staged<P_U32> { using type = uint32_t; };
+template <>
+struct Staged<P_F32> { using type = uint32_t; };
+
+// 64-bit integer add to a shared word as two 32-bit ones (the carry follows
+// from the low half's old value): the 32-bit adds are native, a 64-bit one is
+// a compare-and-swap loop.
+__device__ __forceinline__ void shared_add_i64(uint64_t* p, uint64_t x)
+{
+  uint32_t* w        = reinterpret_cast<uint32_t*>(p);
+  const uint32_t lo  = static_cast<uint32_t>(x);
+  const uint32_t old = atomicAdd(w, lo);
+  const uint32_t hi  = static_cast<uint32_t>(x >> 32) + (old + lo < old ? 1u : 0u);
+  if (hi != 0) atomicAdd(w + 1, hi);
+}
+
+__device__ __forceinline__ uint64_t shfl_down_u64(uint64_t v, int o)
+{
+  return static_cast<uint64_t>(__shfl_down_sync(kFull, static_cast<unsigned long long>(v), o));
+}
+
+// Folds one chunk (staged positions p0 .. p0 + len) of a channel of physical
+// type PT in registers and merges it into slot s of the CTA table at `smem`;
+// `uniform`: the warp's 32 chunks are all of slot s (all 32 lanes call it).
+// The VAR sums are relative to the slot's shift, which the first chunk with a
+// valid non-NaN value records.  Nulls are folded as identities.
+template <int PT>
+__device__ __forceinline__ void fold_chunk(const Channel& ch, unsigned char* smem, const SmemLayout& sl,
+                                           uint32_t val_off, uint32_t ok_off, uint32_t p0, uint32_t len, uint32_t s,
+                                           bool uniform, uint32_t lanes, int32_t* status)
+{
+  constexpr bool kFloat = PT == P_F32 || PT == P_F64;
+  constexpr bool kM64   = PT == P_I64 || PT == P_U64 || PT == P_F64;
+  using T               = typename Staged<PT>::type;
+  using M               = typename std::conditional<kM64, uint64_t, uint32_t>::type;
+  const T* vals         = reinterpret_cast<const T*>(smem + val_off) + p0;
+  const uint8_t* oks    = ok_off ? smem + ok_off + p0 : nullptr;
+  const uint32_t roles  = chan_roles(ch);
+
+  uint32_t cnt = 0;
+  M mn = static_cast<M>(~0ULL), mx = 0;
+  uint64_t sum = 0, sq = 0, prod = 1;  // integer channels
+  double fsum = 0.0, fsq = 0.0, fprod = 1.0, s2 = 0.0, s1 = 0.0, K = 0.0;
+  if (roles & R_VAR) {
+    uint64_t* kp = reinterpret_cast<uint64_t*>(smem + sl.acc_off[ch.a_k]) + s;
+    uint64_t kb  = *kp;
+    if (kb == kShiftUnset) {
+      for (uint32_t j = 0; j < len; ++j) {
+        if (oks != nullptr && !oks[j]) continue;
+        const double x = as_f64(vals[j], PT);
+        if (x != x) continue;
+        const uint64_t xb = static_cast<uint64_t>(__double_as_longlong(x));
+        kb = atomicCAS(reinterpret_cast<unsigned long long*>(kp), static_cast<unsigned long long>(kShiftUnset),
+                       static_cast<unsigned long long>(xb));
+        if (kb == kShiftUnset) kb = xb;
+        break;
+      }
+    }
+    K = __longlong_as_double(static_cast<long long>(kb));
+    __syncwarp(lanes);
+  }
+  for (uint32_t j0 = 0; j0 < len; j0 += 4) {
+    uint64_t b[4];
+    bool ok[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t j = j0 + i;
+      ok[i]            = j < len;
+      b[i]             = ok[i] ? static_cast<uint64_t>(vals[j]) : 0;
+      if (oks != nullptr) ok[i] = ok[i] && oks[j] != 0;
+      cnt += ok[i] ? 1u : 0u;
+    }
+    if (roles & (R_MIN | R_MAX)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (roles & R_MIN) mn = min(mn, ok[i] ? static_cast<M>(enc_minmax(b[i], PT, true)) : static_cast<M>(~0ULL));
+        if (roles & R_MAX) mx = max(mx, ok[i] ? static_cast<M>(enc_minmax(b[i], PT, false)) : static_cast<M>(0));
+      }
+    }
+    if constexpr (kFloat) {
+      double x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = ok[i] ? as_f64(b[i], PT) : 0.0;
+      if (roles & R_SUM) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fsum += x[i];
+      }
+      if (roles & R_VAR) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double d = ok[i] ? x[i] - K : 0.0;
+          s2 += d * d;
+          s1 += d;
+        }
+      }
+      if (roles & R_SQ) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fsq += x[i] * x[i];
+      }
+      if (roles & R_PROD) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fprod *= ok[i] ? x[i] : 1.0;
+      }
+    } else {
+      int64_t x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = ok[i] ? as_i64(b[i], PT) : 0;
+      if (roles & R_SUM) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum += static_cast<uint64_t>(x[i]);
+      }
+      if (roles & R_VAR) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const double xf = PT == P_U64 ? static_cast<double>(static_cast<uint64_t>(x[i])) : static_cast<double>(x[i]);
+          const double d  = ok[i] ? xf - K : 0.0;
+          s2 += d * d;
+        }
+      }
+      if (roles & R_SQ) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq += static_cast<uint64_t>(x[i]) * static_cast<uint64_t>(x[i]);
+      }
+      if (roles & R_PROD) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) prod *= ok[i] ? static_cast<uint64_t>(x[i]) : 1ULL;
+      }
+    }
+  }
+  __syncwarp(lanes);
+  if (uniform) {
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+      cnt += __shfl_down_sync(kFull, cnt, o);
+      if (roles & R_MIN) {
+        if constexpr (kM64) mn = min(mn, static_cast<M>(shfl_down_u64(mn, o)));
+        else mn = min(mn, static_cast<M>(__shfl_down_sync(kFull, mn, o)));
+      }
+      if (roles & R_MAX) {
+        if constexpr (kM64) mx = max(mx, static_cast<M>(shfl_down_u64(mx, o)));
+        else mx = max(mx, static_cast<M>(__shfl_down_sync(kFull, mx, o)));
+      }
+      if constexpr (kFloat) {
+        if (roles & R_SUM) fsum += __shfl_down_sync(kFull, fsum, o);
+        if (roles & R_SQ) fsq += __shfl_down_sync(kFull, fsq, o);
+        if (roles & R_PROD) fprod *= __shfl_down_sync(kFull, fprod, o);
+      } else {
+        if (roles & R_SUM) sum += shfl_down_u64(sum, o);
+        if (roles & R_SQ) sq += shfl_down_u64(sq, o);
+        if (roles & R_PROD) prod *= shfl_down_u64(prod, o);
+      }
+      if (roles & R_VAR) {
+        s2 += __shfl_down_sync(kFull, s2, o);
+        s1 += __shfl_down_sync(kFull, s1, o);
+      }
+    }
+  }
+  // the lanes meet again after every compare-and-swap loop (floating adds), or
+  // the rest of the merge and the next channel would run apart
+  const bool mine = cnt != 0 && (!uniform || (threadIdx.x & 31) == 0);
+  if (mine) {
+    if (ch.a_cnt >= 0) atomicAdd(reinterpret_cast<uint32_t*>(smem + sl.acc_off[ch.a_cnt]) + s, cnt);
+    // a slot's extremes settle early: most chunks only read them
+    if (roles & R_MIN) {
+      M* p = reinterpret_cast<M*>(smem + sl.acc_off[ch.a_min]) + s;
+      if constexpr (kM64) {
+        if (mn < *p) atomicMin(reinterpret_cast<unsigned long long*>(p), static_cast<unsigned long long>(mn));
+      } else {
+        if (mn < *p) atomicMin(reinterpret_cast<uint32_t*>(p), static_cast<uint32_t>(mn));
+      }
+    }
+    if (roles & R_MAX) {
+      M* p = reinterpret_cast<M*>(smem + sl.acc_off[ch.a_max]) + s;
+      if constexpr (kM64) {
+        if (mx > *p) atomicMax(reinterpret_cast<unsigned long long*>(p), static_cast<unsigned long long>(mx));
+      } else {
+        if (mx > *p) atomicMax(reinterpret_cast<uint32_t*>(p), static_cast<uint32_t>(mx));
+      }
+    }
+    if constexpr (!kFloat) {
+      if (roles & R_SUM) shared_add_i64(reinterpret_cast<uint64_t*>(smem + sl.acc_off[ch.a_sum]) + s, sum);
+      if (roles & R_SQ) shared_add_i64(reinterpret_cast<uint64_t*>(smem + sl.acc_off[ch.a_sq]) + s, sq);
+    }
+  }
+  __syncwarp(lanes);
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  if constexpr (kFloat) {
+    if (roles & R_SUM) {
+      if (mine) atomicAdd(reinterpret_cast<double*>(smem + sl.acc_off[ch.a_sum]) + s, fsum);
+      __syncwarp(lanes);
+    }
+    if (roles & R_SQ) {
+      if (mine) atomicAdd(reinterpret_cast<double*>(smem + sl.acc_off[ch.a_sq]) + s, fsq);
+      __syncwarp(lanes);
+    }
+    if (roles & R_PROD) {
+      if (mine) mul_cas_f64<Shared>(base + sl.acc_off[ch.a_prod] + s * 8, fprod, status);
+      __syncwarp(lanes);
+    }
+    if (roles & R_VAR) {
+      if (mine) atomicAdd(reinterpret_cast<double*>(smem + sl.acc_off[ch.a_s1]) + s, s1);
+      __syncwarp(lanes);
+    }
+  } else if (roles & R_PROD) {
+    if (mine) mul_cas_i64<Shared>(base + sl.acc_off[ch.a_prod] + s * 8, static_cast<int64_t>(prod), status);
+    __syncwarp(lanes);
+  }
+  if (roles & R_VAR) {
+    if (mine) atomicAdd(reinterpret_cast<double*>(smem + sl.acc_off[ch.a_s2]) + s, s2);
+    __syncwarp(lanes);
+  }
+}
+
+// The rows q0 .. q0 + kBatch - 1 of a thread that lie in its tile (`per` rows
+// a thread) and below n, as bits; r0 is row q0.
+__device__ __forceinline__ uint32_t in_tile(int q0, int per, int64_t r0, int step, int64_t n)
+{
+  uint32_t m = 0;
+#pragma unroll
+  for (int q = 0; q < kBatch; ++q)
+    if (q0 + q < per && r0 + q * step < n) m |= 1u << q;
+  return m;
+}
+
+// The listed rows of a tile: straight into the global table.
 template <int NW, bool PART>
-__global__ void __launch_bounds__(kTiledBlock, 2) k_agg_tiled(const __grid_constant__ Plan plan,
-                                                           const __grid_constant__ TableRef t,
-                                                           const __grid_constant__ SmemLayout sl,
-                                                           const __grid_constant__ TiledLayout tl, int64_t n,
-                                                           const __grid_constant__ PartBufs pb,
-                                                           const uint32_t* n_part, uint32_t smem_probes,
-                                                           uint32_t max_probes)
+__device__ __noinline__ void spill_rows(const Plan& plan, const TableRef& t, const PartBufs& pb, const uint16_t* list,
+                                        uint32_t n, int64_t t0, uint32_t max_probes)
+{
+  const Level<Global> G = global_level(t);
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    const int64_t r = t0 + list[i];
+    uint64_t k[NW];
+    if constexpr (PART) PartSource{&pb}.key<NW>(r, k);
+    else pack_key<NW>(plan.key, r, k);
+    const int64_t g = global_slot<NW>(t, k, max_probes);
+    if (g < 0) continue;
+    if constexpr (PART) accumulate_row_from<Global>(plan, PartSource{&pb}, G, g, r, t.status);
+    else accumulate_row<Global>(plan, G, g, r, t.status);
+  }
+}
+
+template <int NW, bool PART, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) k_agg_tiled(const __grid_constant__ Plan plan,
+                                                               const __grid_constant__ TableRef t,
+                                                               const __grid_constant__ SmemLayout sl,
+                                                               const __grid_constant__ TiledLayout tl, int64_t n,
+                                                               const __grid_constant__ PartBufs pb,
+                                                               const uint32_t* n_part, uint32_t smem_probes,
+                                                               uint32_t max_probes)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  using BlockScan = cub::BlockScan<uint32_t, kTiledBlock>;
-  __shared__ typename BlockScan::TempStorage scan_tmp;
-  __shared__ uint32_t s_special;
-  const uint32_t S     = sl.slots;
-  const int tile_rows  = tl.tile_rows;
-  const int per        = tile_rows / kTiledBlock;
-  uint64_t* skeys      = reinterpret_cast<uint64_t*>(smem + sl.keys_off);
-  uint32_t* srows      = reinterpret_cast<uint32_t*>(smem + sl.rows_off);
-  uint32_t* cnt        = reinterpret_cast<uint32_t*>(smem + tl.cnt_off);
-  uint32_t* off        = reinterpret_cast<uint32_t*>(smem + tl.off_off);
-  uint32_t* coff       = reinterpret_cast<uint32_t*>(smem + tl.coff_off);
-  uint16_t* cslot      = reinterpret_cast<uint16_t*>(smem + tl.cslot_off);
-  uint16_t* perm       = reinterpret_cast<uint16_t*>(smem + tl.perm_off);
-  uint64_t* vals       = reinterpret_cast<uint64_t*>(smem + tl.vals_off);
-  uint8_t* valid       = smem + tl.valid_off;
-  const uint32_t base  = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
-  const uint32_t keys  = base + sl.keys_off;
+  constexpr int kWarps = BLOCK / 32;
+  __shared__ uint32_t s_warp[kWarps];
+  __shared__ uint32_t s_nspill;
+  const uint32_t S    = sl.slots;
+  const int tile_rows = tl.tile_rows;
+  const int per       = tile_rows / BLOCK;
+  const int lane      = threadIdx.x & 31;
+  const int warp      = threadIdx.x >> 5;
+  uint64_t* skeys     = reinterpret_cast<uint64_t*>(smem + sl.keys_off);
+  uint32_t* srows     = reinterpret_cast<uint32_t*>(smem + sl.rows_off);
+  uint32_t* cnt       = reinterpret_cast<uint32_t*>(smem + tl.cnt_off);
+  uint32_t* oc        = reinterpret_cast<uint32_t*>(smem + tl.oc_off);
+  uint32_t* rec       = reinterpret_cast<uint32_t*>(smem + tl.rec_off);
+  uint16_t* cslot     = reinterpret_cast<uint16_t*>(smem + tl.cslot_off);
+  uint16_t* spill     = reinterpret_cast<uint16_t*>(smem + tl.spill_off);
+  const uint32_t keys_sa = static_cast<uint32_t>(__cvta_generic_to_shared(smem)) + sl.keys_off;
 
   // identity fill, counts zeroed
-  for (uint32_t s = threadIdx.x; s <= S; s += blockDim.x) {
+  for (uint32_t s = threadIdx.x; s <= S; s += BLOCK) {
 #pragma unroll
     for (int w = 0; w < NW; ++w) skeys[s * NW + w] = kEmptyWord;
     srows[s] = 0;
     cnt[s]   = 0;
-    for (int a = 0; a < plan.acc.nacc; ++a) {
-      const uint64_t id = identity_bits(plan.acc.kind[a]);
-      if (acc_bytes(plan.acc.kind[a]) == 4) reinterpret_cast<uint32_t*>(smem + sl.acc_off[a])[s] = static_cast<uint32_t>(id);
-      else reinterpret_cast<uint64_t*>(smem + sl.acc_off[a])[s] = id;
+  }
+  for (int a = 0; a < plan.acc.nacc; ++a) {
+    const uint64_t id = identity_bits(plan.acc.kind[a]);
+    if (acc_bytes(plan.acc.kind[a]) == 4) {
+      uint32_t* p = reinterpret_cast<uint32_t*>(smem + sl.acc_off[a]);
+      for (uint32_t s = threadIdx.x; s <= S; s += BLOCK) p[s] = static_cast<uint32_t>(id);
+    } else {
+      uint64_t* p = reinterpret_cast<uint64_t*>(smem + sl.acc_off[a]);
+      for (uint32_t s = threadIdx.x; s <= S; s += BLOCK) p[s] = id;
     }
   }
-  if (threadIdx.x == 0) s_special = 0;
+  if (threadIdx.x == 0) s_nspill = 0;
   __syncthreads();
 
-  const Level<Global> G = global_level(t);
-  const RowSource src{&plan};
-  const PartSource psrc{&pb};
   if constexpr (PART) n = *n_part;
   const int64_t ntiles     = (n + tile_rows - 1) / tile_rows;
   const int64_t tile_begin = PART ? ntiles * blockIdx.x / gridDim.x : blockIdx.x;
   const int64_t tile_end   = PART ? ntiles * (blockIdx.x + 1) / gridDim.x : ntiles;
   const int64_t tile_step  = PART ? 1 : gridDim.x;
+  const uint32_t slots_per = (S + 1 + BLOCK - 1) / BLOCK;  // slots scanned by one thread
   for (int64_t tile = tile_begin; tile < tile_end; tile += tile_step) {
     const int64_t t0 = tile * tile_rows;
-    // 1a. keys (this thread's rows threadIdx.x + q * kTiledBlock)
-    uint64_t k[kTiledPer][NW];
-    bool kept[kTiledPer];
-#pragma unroll
-    for (int q = 0; q < kTiledPer; ++q) {
-      const int64_t r = t0 + threadIdx.x + q * kTiledBlock;
-      if constexpr (PART) kept[q] = q < per && r < n && psrc.key<NW>(r, k[q]);
-      else kept[q] = q < per && r < n && pack_key<NW>(plan.key, r, k[q]);
-    }
-    // 1b. values and validity of the kept rows, staged channel by channel
-    for (int c = 0; c < plan.nchan; ++c) {
-      const Channel& ch = plan.chan[c];
-      uint64_t* cv      = vals + static_cast<size_t>(c) * tile_rows;
-      uint8_t* cvv      = valid + static_cast<size_t>(c) * tile_rows;
+    // 1. slot and rank of each row (kNoRec: no row, excluded, or listed)
+#pragma unroll 1
+    for (int q0 = 0; q0 < per; q0 += kBatch) {
+      const int64_t r0 = t0 + threadIdx.x + q0 * BLOCK;
+      uint32_t kept    = in_tile(q0, per, r0, BLOCK, n);
+      uint64_t k[kBatch][NW];
       if constexpr (PART) {
-        const PartCol& pc = pb.col[c];
-        uint64_t b[kTiledPer];
-        bool v[kTiledPer];
 #pragma unroll
-        for (int q = 0; q < kTiledPer; ++q) {
-          const int64_t i = t0 + threadIdx.x + q * kTiledBlock;
-          b[q]            = kept[q] ? load_bits(pc.vals, i, pc.width) : 0;
-          v[q]            = kept[q] && (pc.valid == nullptr || __ldg(pc.valid + i) != 0);
-        }
+        for (int q = 0; q < kBatch; ++q)
 #pragma unroll
-        for (int q = 0; q < kTiledPer; ++q) {
-          if (!kept[q]) continue;
-          const int li = threadIdx.x + q * kTiledBlock;
-          cv[li]       = v[q] ? b[q] : 0;
-          cvv[li]      = v[q] ? 1 : 0;
-        }
-      } else if (ch.dict_data == nullptr) {
-        const int w = pt_width(ch.ptype);
-        uint64_t b[kTiledPer];
-        bool v[kTiledPer];
-#pragma unroll
-        for (int q = 0; q < kTiledPer; ++q) {
-          const int64_t i = t0 + threadIdx.x + q * kTiledBlock + ch.offset;
-          b[q]            = kept[q] ? load_bits(ch.data, i, w) : 0;
-          v[q]            = kept[q] && bit_valid(ch.mask, i);
-        }
-#pragma unroll
-        for (int q = 0; q < kTiledPer; ++q) {
-          if (!kept[q]) continue;
-          const int li = threadIdx.x + q * kTiledBlock;
-          cv[li]       = v[q] ? b[q] : 0;
-          cvv[li]      = v[q] ? 1 : 0;
-        }
+          for (int w = 0; w < NW; ++w) k[q][w] = ((kept >> q) & 1u) ? __ldg(pb.keys[w] + r0 + q * BLOCK) : 0;
       } else {
-        for (int q = 0; q < kTiledPer; ++q) {
-          if (!kept[q]) continue;
-          const int li = threadIdx.x + q * kTiledBlock;
-          uint64_t b   = 0;
-          const bool v = src.value(c, t0 + li, b, t.status);
-          cv[li]       = v ? b : 0;
-          cvv[li]      = v ? 1 : 0;
-        }
+        kept = pack_rows<kBatch, NW>(plan.key, PlanKeyBufs{&plan.key}, r0, BLOCK, kept, k);
+      }
+      uint32_t slot[kBatch];
+      const uint32_t found = find_slots<kBatch, NW>(skeys, keys_sa, S - 1, kept, k, smem_probes, slot);
+      if (__any_sync(kFull, found != kept)) {
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+          if (((kept & ~found) >> q) & 1u)
+            spill[atomicAdd(&s_nspill, 1u)] = static_cast<uint16_t>(threadIdx.x + (q0 + q) * BLOCK);
+        __syncwarp();
+      }
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        if (q0 + q >= per) break;
+        rec[threadIdx.x + (q0 + q) * BLOCK] =
+          ((found >> q) & 1u) ? (slot[q] << 16) | atomicAdd(cnt + slot[q], 1u) : kNoRec;
       }
     }
-    // 1c. slot and rank of every kept row (kNoRec: no row, key excluded, or
-    //     sent to the global table)
-    uint32_t rec[kTiledPer];
-#pragma unroll
-    for (int q = 0; q < kTiledPer; ++q) {
-      rec[q] = kNoRec;
-      if (!kept[q]) continue;
-      int64_t s;
-      if (key_is_empty<NW>(k[q])) {
-        s = S;
-        if (s_special == 0) s_special = 1;
-      } else {
-        s = find_or_insert<Shared, NW>(keys, S - 1, k[q], hash_key<NW>(k[q]), smem_probes);
-      }
-      if (s >= 0) {
-        const uint32_t rank = atomicAdd(cnt + s, 1u);
-        rec[q]              = (static_cast<uint32_t>(s) << 16) | rank;
-      } else {
-        const int64_t g = global_slot<NW>(t, k[q], max_probes);
-        const int64_t r = t0 + threadIdx.x + q * kTiledBlock;
-        if (g >= 0) {
-          if constexpr (PART) accumulate_row_from<Global>(plan, psrc, G, g, r, t.status);
-          else accumulate_row<Global>(plan, G, g, r, t.status);
-        }
-      }
+    // the first values load across the scan
+    uint64_t v[kBatch];
+    uint32_t ok = 0;
+    if (plan.nchan > 0 && (PART || plan.chan[0].dict_data == nullptr)) {
+      const int64_t r0 = t0 + threadIdx.x;
+      ok               = channel_rows<PART>(plan, pb, 0, r0, BLOCK, in_tile(0, per, r0, BLOCK, n), v);
     }
     __syncthreads();
-    // 2. first position of each slot's rows; the rows listed in slot order
-    {
-      uint32_t c[kScanPer];
-#pragma unroll
-      for (int q = 0; q < kScanPer; ++q) {
-        const uint32_t s = threadIdx.x * kScanPer + q;
-        c[q]             = s <= S ? cnt[s] : 0u;
-      }
-      BlockScan(scan_tmp).ExclusiveSum(c, c);
-#pragma unroll
-      for (int q = 0; q < kScanPer; ++q) {
-        const uint32_t s = threadIdx.x * kScanPer + q;
-        if (s <= S) off[s] = c[q];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kTiledPer; ++q)
-      if (rec[q] != kNoRec)
-        perm[off[rec[q] >> 16] + (rec[q] & 0xffffu)] = static_cast<uint16_t>(threadIdx.x + q * kTiledBlock);
-    __syncthreads();
-    // 3a. one thread per occupied slot: row count, and the VAR shift of each
-    //     channel whose slot has none yet (the group's first valid non-NaN
-    //     value in this tile), so that every chunk below folds against it
-    uint32_t nchunk[kScanPer];
-#pragma unroll
-    for (int q = 0; q < kScanPer; ++q) {
-      const uint32_t s = threadIdx.x * kScanPer + q;
+    const uint32_t nspill = s_nspill;
+    // 2. (chunks << 16 | rows) scanned over the slots
+    uint32_t sum = 0;
+    for (uint32_t q = 0; q < slots_per; ++q) {
+      const uint32_t s = threadIdx.x * slots_per + q;
       const uint32_t c = s <= S ? cnt[s] : 0u;
-      nchunk[q]        = (c + kChunk - 1) / kChunk;
-      if (c == 0) continue;
-      srows[s] += c;
-      for (int ch = 0; ch < plan.nchan; ++ch) {
-        const Channel& chan = plan.chan[ch];
-        if (chan.a_k < 0) continue;
-        uint64_t* kp = reinterpret_cast<uint64_t*>(smem + sl.acc_off[chan.a_k]) + s;
-        if (*kp != kShiftUnset) continue;
-        const uint64_t* cv = vals + static_cast<size_t>(ch) * tile_rows;
-        const uint8_t* cvv = valid + static_cast<size_t>(ch) * tile_rows;
-        for (uint32_t j = 0; j < c; ++j) {
-          const uint32_t li = perm[off[s] + j];
-          if (!cvv[li]) continue;
-          const double xf = as_f64(cv[li], chan.ptype);
-          if (xf != xf) continue;
-          *kp = static_cast<uint64_t>(__double_as_longlong(xf));
-          break;
-        }
-      }
+      sum += c | (((c + kChunk - 1) / kChunk) << 16);
     }
-    // chunks of at most kChunk rows of one group: first chunk of each slot
-    uint32_t total_chunks;
-    BlockScan(scan_tmp).ExclusiveSum(nchunk, nchunk, total_chunks);
-    __syncthreads();
+    uint32_t incl = sum;
 #pragma unroll
-    for (int q = 0; q < kScanPer; ++q) {
-      const uint32_t s = threadIdx.x * kScanPer + q;
-      if (s > S) continue;
-      const uint32_t n_s = (cnt[s] + kChunk - 1) / kChunk;
-      for (uint32_t j = 0; j < n_s; ++j) cslot[nchunk[q] + j] = static_cast<uint16_t>(s);
-      if (n_s > 0) coff[s] = nchunk[q];
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += x;
     }
+    if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
-    // 3b. every thread folds chunks in registers and merges each into its
-    //     group's slot with shared atomics (a few chunks per group)
-    const Level<Shared> L{base, &sl};
-    for (uint32_t ci = threadIdx.x; ci < total_chunks; ci += blockDim.x) {
-      const uint32_t s     = cslot[ci];
-      const uint32_t j0    = (ci - coff[s]) * kChunk;
-      const uint32_t first = off[s] + j0;
-      const uint32_t len   = min(static_cast<uint32_t>(kChunk), cnt[s] - j0);
-      for (int ch = 0; ch < plan.nchan; ++ch) {
-        const Channel& chan = plan.chan[ch];
-        const uint64_t* cv  = vals + static_cast<size_t>(ch) * tile_rows;
-        const uint8_t* cvv  = valid + static_cast<size_t>(ch) * tile_rows;
-        ChanAcc A;
-        chan_acc_init(A);
-        if (chan.a_k >= 0) A.k = reinterpret_cast<const uint64_t*>(smem + sl.acc_off[chan.a_k])[s];
-#define GBX_FOLD_CHUNK(P) fold_chunk<P>(chan, cv, cvv, perm + first, len, A)
-        switch (chan.ptype) {
-          case P_I8: GBX_FOLD_CHUNK(P_I8); break;
-          case P_I16: GBX_FOLD_CHUNK(P_I16); break;
-          case P_I32: GBX_FOLD_CHUNK(P_I32); break;
-          case P_I64: GBX_FOLD_CHUNK(P_I64); break;
-          case P_U8: GBX_FOLD_CHUNK(P_U8); break;
-          case P_U16: GBX_FOLD_CHUNK(P_U16); break;
-          case P_U32: GBX_FOLD_CHUNK(P_U32); break;
-          case P_U64: GBX_FOLD_CHUNK(P_U64); break;
-          case P_F32: GBX_FOLD_CHUNK(P_F32); break;
-          case P_F64: GBX_FOLD_CHUNK(P_F64); break;
-          default: GBX_FOLD_CHUNK(P_BOOL); break;
+    uint32_t total;
+    {
+      const uint32_t w = lane < kWarps ? s_warp[lane] : 0u;
+      uint32_t wi      = w;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(kFull, wi, o);
+        if (lane >= o) wi += x;
+      }
+      total        = __shfl_sync(kFull, wi, 31);
+      uint32_t run = __shfl_sync(kFull, wi - w, warp) + incl - sum;
+      for (uint32_t q = 0; q < slots_per; ++q) {
+        const uint32_t s = threadIdx.x * slots_per + q;
+        if (s > S) break;
+        const uint32_t c  = cnt[s];
+        const uint32_t nc = (c + kChunk - 1) / kChunk;
+        oc[s]             = run;
+        if (c != 0) {
+          srows[s] += c;
+          cnt[s] = 0;
+          for (uint32_t j = 0; j < nc; ++j) cslot[(run >> 16) + j] = static_cast<uint16_t>(s);
         }
-#undef GBX_FOLD_CHUNK
-        merge_partial(chan, A, L, s, t.status);
+        run += c | (nc << 16);
+      }
+      if (threadIdx.x == 0) {
+        oc[S + 1] = total;
+        s_nspill  = 0;
       }
     }
     __syncthreads();
-    for (uint32_t s = threadIdx.x; s <= S; s += blockDim.x) cnt[s] = 0;
+    // 3. the values, group by group; the next values load while these are
+    //    stored
+#pragma unroll 1
+    for (int q0 = 0; q0 < per; q0 += kBatch) {
+      const int64_t r0 = t0 + threadIdx.x + q0 * BLOCK;
+      uint32_t pos[kBatch];
+      uint32_t rows = 0;
+#pragma unroll
+      for (int q = 0; q < kBatch; ++q) {
+        pos[q] = q0 + q < per ? rec[threadIdx.x + (q0 + q) * BLOCK] : kNoRec;
+        if (pos[q] != kNoRec) {
+          rows |= 1u << q;
+          pos[q] = (oc[pos[q] >> 16] & 0xffffu) + (pos[q] & 0xffffu);
+        }
+      }
+#pragma unroll 1
+      for (int c = 0; c < plan.nchan; ++c) {
+        if (!PART && plan.chan[c].dict_data != nullptr) ok = dict_rows(plan, c, r0, BLOCK, rows, v, t.status);
+        uint64_t vn[kBatch] = {};
+        uint32_t okn        = 0;
+        {
+          const bool last = c + 1 == plan.nchan;
+          const int cn    = last ? 0 : c + 1;
+          const int qn    = last ? q0 + kBatch : q0;
+          if (qn < per && (PART || plan.chan[cn].dict_data == nullptr)) {
+            const int64_t rn = t0 + threadIdx.x + qn * BLOCK;
+            okn              = channel_rows<PART>(plan, pb, cn, rn, BLOCK, in_tile(qn, per, rn, BLOCK, n), vn);
+          }
+        }
+        unsigned char* dst = smem + tl.val_off[c];
+#define GBX_STAGE(T)                                                                           \
+  _Pragma("unroll") for (int q = 0; q < kBatch; ++q) if ((rows >> q) & 1u)                     \
+    reinterpret_cast<T*>(dst)[pos[q]] = static_cast<T>(v[q]);                                  \
+  break;
+        switch (pt_width(plan.chan[c].ptype)) {
+          case 1: GBX_STAGE(uint8_t)
+          case 2: GBX_STAGE(uint16_t)
+          case 4: GBX_STAGE(uint32_t)
+          default: GBX_STAGE(uint64_t)
+        }
+#undef GBX_STAGE
+        if (tl.ok_off[c] != 0) {
+          uint8_t* d = smem + tl.ok_off[c];
+#pragma unroll
+          for (int q = 0; q < kBatch; ++q)
+            if ((rows >> q) & 1u) d[pos[q]] = (ok >> q) & 1u;
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) v[q] = vn[q];
+        ok = okn;
+      }
+    }
+    if (nspill != 0) spill_rows<NW, PART>(plan, t, pb, spill, nspill, t0, max_probes);
     __syncthreads();
+    // 4. one chunk per thread
+    const uint32_t nchunks = total >> 16;
+    for (uint32_t c0 = static_cast<uint32_t>(warp) * 32; c0 < nchunks; c0 += BLOCK) {
+      const uint32_t ci  = c0 + lane;
+      const bool active  = ci < nchunks;
+      const uint32_t s   = cslot[active ? ci : c0];
+      const uint32_t o0  = oc[s];
+      const uint32_t j0  = (ci - (o0 >> 16)) * kChunk;
+      const uint32_t p0  = (o0 & 0xffffu) + j0;
+      const uint32_t len = min(static_cast<uint32_t>(kChunk), (oc[s + 1] & 0xffffu) - p0);
+      const uint32_t s0  = __shfl_sync(kFull, s, 0);
+      const uint32_t lanes = __ballot_sync(kFull, active);
+      const bool uniform   = __all_sync(kFull, active && s == s0);
+      if (!active) continue;
+      for (int c = 0; c < plan.nchan; ++c) {
+        const Channel& ch = plan.chan[c];
+#define GBX_FOLD(P) fold_chunk<P>(ch, smem, sl, tl.val_off[c], tl.ok_off[c], p0, len, s, uniform, lanes, t.status); break;
+        switch (ch.ptype) {
+          case P_I8: GBX_FOLD(P_I8)
+          case P_I16: GBX_FOLD(P_I16)
+          case P_I32: GBX_FOLD(P_I32)
+          case P_I64: GBX_FOLD(P_I64)
+          case P_U8: GBX_FOLD(P_U8)
+          case P_U16: GBX_FOLD(P_U16)
+          case P_U32: GBX_FOLD(P_U32)
+          case P_U64: GBX_FOLD(P_U64)
+          case P_F32: GBX_FOLD(P_F32)
+          case P_F64: GBX_FOLD(P_F64)
+          default: GBX_FOLD(P_BOOL)
+        }
+#undef GBX_FOLD
+      }
+    }
+    // no barrier here: the next tile's ranking touches only the keys and
+    // `cnt`, and its scan waits for every thread to have left this fold
   }
-
+  __syncthreads();
   // merge the CTA's table into the global one
-  for (uint32_t s = threadIdx.x; s <= S; s += blockDim.x) {
+  const Level<Shared> L{static_cast<uint32_t>(__cvta_generic_to_shared(smem)), &sl};
+  const Level<Global> G = global_level(t);
+  for (uint32_t s = threadIdx.x; s <= S; s += BLOCK) {
+    if (srows[s] == 0) continue;
     uint64_t k[NW];
 #pragma unroll
     for (int w = 0; w < NW; ++w) k[w] = skeys[s * NW + w];
-    const bool occupied = (s < S) ? !key_is_empty<NW>(k) : (s_special != 0);
-    if (!occupied) continue;
     const int64_t g = global_slot<NW>(t, k, max_probes);
-    if (g >= 0) merge_slot<Shared>(plan, Level<Shared>{base, &sl}, s, G, g, t.status);
+    if (g >= 0) merge_slot<Shared>(plan, L, s, G, g, t.status);
   }
 }
 
-template <int NW, bool PART>
-cudaError_t launch_tiled_nw(const Plan& p, const TableRef& t, const SmemLayout& sl, const TiledLayout& tl,
-                            int64_t n, const PartBufs& pb, const uint32_t* n_part, int num_sms,
-                            uint32_t smem_probes, uint32_t max_probes, cudaStream_t st)
+template <int NW, bool PART, int BLOCK>
+cudaError_t launch_tiled_as(const Plan& p, const TableRef& t, const SmemLayout& sl, const TiledLayout& tl, int64_t n,
+                            const PartBufs& pb, const uint32_t* n_part, int num_sms, uint32_t smem_probes,
+                            uint32_t max_probes, cudaStream_t st)
 {
-  const void* fn = reinterpret_cast<const void*>(k_agg_tiled<NW, PART>);
+  const void* fn = reinterpret_cast<const void*>(k_agg_tiled<NW, PART, BLOCK>);
   cudaError_t e  = ensure_dynamic_smem(fn, tl.total);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_agg_tiled<NW, PART>, kTiledBlock, tl.total)) !=
-      cudaSuccess)
-    return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int64_t ntiles = (n + tl.tile_rows - 1) / tl.tile_rows;
-  const int grid       = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(ntiles, int64_t(num_sms) * per_sm)));
-  k_agg_tiled<NW, PART><<<grid, kTiledBlock, tl.total, st>>>(p, t, sl, tl, n, pb, n_part, smem_probes, max_probes);
+  const int64_t cap    = static_cast<int64_t>(num_sms) * (1024 / BLOCK);
+  const int grid       = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(ntiles, cap)));
+  k_agg_tiled<NW, PART, BLOCK><<<grid, BLOCK, tl.total, st>>>(p, t, sl, tl, n, pb, n_part, smem_probes, max_probes);
   return cudaGetLastError();
+}
+
+template <bool PART>
+cudaError_t launch_tiled(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, const PartBufs& pb,
+                         const uint32_t* n_part, int num_sms, uint32_t smem_probes, uint32_t max_probes,
+                         cudaStream_t st)
+{
+  TiledLayout tl = pick_tiled_layout(sl, p);
+  if (tl.tile_rows == 0) return cudaErrorInvalidValue;
+  if (n <= 0) return cudaSuccess;
+  // few rows: tiles small enough that every SM gets one
+  const int64_t ctas = static_cast<int64_t>(num_sms) * (1024 / tl.block);
+  const int64_t want = (n + ctas * tl.block - 1) / (ctas * tl.block) * tl.block;
+  if (want < tl.tile_rows) tl = tiled_layout(sl, p, tl.block, static_cast<int>(want));
+  const bool one = p.key.nwords == 1;
+  if (tl.block == 512)
+    return one ? launch_tiled_as<1, PART, 512>(p, t, sl, tl, n, pb, n_part, num_sms, smem_probes, max_probes, st)
+               : launch_tiled_as<2, PART, 512>(p, t, sl, tl, n, pb, n_part, num_sms, smem_probes, max_probes, st);
+  return one ? launch_tiled_as<1, PART, 1024>(p, t, sl, tl, n, pb, n_part, num_sms, smem_probes, max_probes, st)
+             : launch_tiled_as<2, PART, 1024>(p, t, sl, tl, n, pb, n_part, num_sms, smem_probes, max_probes, st);
 }
 
 }  // namespace
 
-bool tiled_fits(const SmemLayout& sl, int nchan)
+bool tiled_fits(const SmemLayout& sl, const Plan& p, bool two_per_sm)
 {
-  return sl.slots <= static_cast<uint32_t>(kTiledMaxSlots) && pick_tiled_layout(sl, nchan).tile_rows > 0;
+  if (sl.slots > static_cast<uint32_t>(kMaxSlots)) return false;
+  const TiledLayout tl = pick_tiled_layout(sl, p);
+  return tl.tile_rows > 0 && (!two_per_sm || tl.block == 512);
 }
 
 cudaError_t launch_agg_tiled(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int num_sms,
                              uint32_t smem_probes, uint32_t max_probes, cudaStream_t st)
 {
-  if (!tiled_fits(sl, p.nchan)) return cudaErrorInvalidValue;
-  if (n <= 0) return cudaSuccess;
-  const TiledLayout tl = pick_tiled_layout(sl, p.nchan);
-  const PartBufs none{};
-  return p.key.nwords == 1 ? launch_tiled_nw<1, false>(p, t, sl, tl, n, none, nullptr, num_sms, smem_probes, max_probes, st)
-                           : launch_tiled_nw<2, false>(p, t, sl, tl, n, none, nullptr, num_sms, smem_probes, max_probes, st);
+  return launch_tiled<false>(p, t, sl, n, PartBufs{}, nullptr, num_sms, smem_probes, max_probes, st);
 }
 
 cudaError_t launch_agg_tiled_part(const Plan& p, const TableRef& t, const SmemLayout& sl, const PartBufs& in,
                                   const uint32_t* n_rows, int64_t n, int num_sms, uint32_t smem_probes,
                                   uint32_t max_probes, cudaStream_t st)
 {
-  if (!tiled_fits(sl, p.nchan)) return cudaErrorInvalidValue;
-  if (n <= 0) return cudaSuccess;
-  const TiledLayout tl = pick_tiled_layout(sl, p.nchan);
-  return p.key.nwords == 1 ? launch_tiled_nw<1, true>(p, t, sl, tl, n, in, n_rows, num_sms, smem_probes, max_probes, st)
-                           : launch_tiled_nw<2, true>(p, t, sl, tl, n, in, n_rows, num_sms, smem_probes, max_probes, st);
+  return launch_tiled<true>(p, t, sl, n, in, n_rows, num_sms, smem_probes, max_probes, st);
 }
 
 }  // namespace gbx
