@@ -1006,18 +1006,17 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       if (bucket_slots == 0) strategy = GBX_STRATEGY_GLOBAL;
     }
     // Skewed keys: when the keys sampled 4 or more times hold most sampled
-    // rows and fit a CTA table of the streamed-tile kernel, that kernel keeps
+    // rows and fit a CTA table of the tiled kernel, that kernel keeps
     // them in shared memory and sends the rare keys' rows to the global table
     // (a Zipf key whose hottest group holds a fifth of the rows would
     // otherwise serialise the global table's atomics on one slot).
     const double s_heavy = static_cast<double>(h_ctl[32]), s_heavy_rows = static_cast<double>(h_ctl[33]);
     const bool skewed    = h_ctl[0] > 0 && s_heavy_rows >= 0.75 * static_cast<double>(h_ctl[0]);
-    // table of the streamed-tile kernel: twice the heavy keys (one CTA an SM
-    // when it does not fit two)
+    // its table: twice the heavy keys (one CTA an SM when it does not fit two)
     uint32_t stream_slots = 0;
-    if (skewed && plan.key.nwords == 1 && !plan_has_arg(plan)) {
+    if (skewed && !plan_has_arg(plan)) {
       const auto need = static_cast<uint32_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * s_heavy, 64.0))));
-      if (need <= 4096 && stream_fits(plan, make_smem_layout(plan, need))) stream_slots = need;
+      if (need <= 4096 && tiled_fits(make_smem_layout(plan, need), plan)) stream_slots = need;
     }
     bool skew_stream = false;
     if (strategy == GBX_STRATEGY_AUTO) {
@@ -1399,11 +1398,11 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
         int64_t max_grid = (call.n + block * 4 - 1) / (block * 4);
         grid             = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(grid, max_grid)));
         if (skew_stream) {
-          // skewed keys: the streamed-tile kernel keeps the hot keys in shared
+          // skewed keys: the tiled kernel keeps the hot keys in shared
           // memory and sends the rare keys' rows to the global table
           // a short probe: a hot key was inserted early and sits near its home
           // slot; a rare key that misses goes to the global table
-          GBX_CUDA(launch_agg_stream(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 8), max_probes, s));
+          GBX_CUDA(launch_agg_tiled(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 8), max_probes, s));
         } else if (tiled_fits(sl, plan) && !arg_kinds) {
           // few groups: tiles grouped in shared memory before the table is touched
           GBX_CUDA(launch_agg_tiled(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 32), max_probes, s));

@@ -58,12 +58,6 @@ cudaError_t launch_agg_privatized(const Plan& p, const TableRef& t, const SmemLa
 // and a tile's staged values within an SM's shared memory, or within half of
 // it with two_per_sm).
 bool tiled_fits(const SmemLayout& sl, const Plan& p, bool two_per_sm = false);
-// Streamed tiles grouped in shared memory (gbx_stream.cu): one packed key
-// word, no ARGMIN/ARGMAX, a table of at most 4,096 slots.
-bool stream_fits(const Plan& p, const SmemLayout& sl);
-size_t stream_smem_bytes(const Plan& p, const SmemLayout& sl);
-cudaError_t launch_agg_stream(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int num_sms,
-                              uint32_t smem_probes, uint32_t max_probes, cudaStream_t st);
 cudaError_t launch_agg_tiled(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int num_sms,
                              uint32_t smem_probes, uint32_t max_probes, cudaStream_t st);
 // ---- radix-partitioned path
