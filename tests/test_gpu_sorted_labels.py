@@ -1,0 +1,39 @@
+"""The sorted kinds' row labels and NTH_ELEMENT's first / last rows
+(gbx_sort.cu) against the oracle: label tables in shared memory and beyond it,
+the all-ones key, two-word keys, excluded keys, and n = 0 / -1 under both null
+policies beside another n."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cudf_b200._abi import Kind, NullPolicy
+from oracle.oracle import HostCol
+from tests import gbx_testing as T
+
+pytestmark = pytest.mark.gpu
+
+
+def _nth(n, policy):
+    return (Kind.NTH_ELEMENT, n, {"null_policy": policy})
+
+
+@pytest.mark.parametrize("n,groups", [(1, 1), (1023, 7), (70_001, 900), (1_100_000, 12_000), (1_100_003, 13_000)])
+def test_labels_and_ends(n, groups):
+    rng = np.random.default_rng(groups)
+    k = rng.integers(0, groups, n).astype(np.int64) - 1  # -1: the all-ones word
+    v = rng.integers(-1000, 1000, n).astype(np.int64)
+    w = rng.standard_normal(n).astype(np.float32)
+    aggs = [_nth(0, NullPolicy.INCLUDE), _nth(-1, NullPolicy.INCLUDE), _nth(0, NullPolicy.EXCLUDE),
+            _nth(-1, NullPolicy.EXCLUDE), _nth(1, NullPolicy.EXCLUDE)]
+    T.assert_parity([HostCol(k, rng.random(n) >= 0.05)],
+                    [(HostCol(v), [(Kind.NUNIQUE, 0, {"null_policy": NullPolicy.EXCLUDE}), aggs[0], aggs[1]]),
+                     (HostCol(w, rng.random(n) >= 0.4), aggs)])
+
+
+def test_two_word_keys():
+    rng = np.random.default_rng(3)
+    n = 50_000
+    keys = [HostCol(rng.integers(-2, 40, n).astype(np.int64)), HostCol(rng.integers(-1, 9, n).astype(np.int64))]
+    T.assert_parity(keys, [(HostCol(rng.integers(0, 99, n).astype(np.int16)),
+                            [_nth(0, NullPolicy.INCLUDE), _nth(-1, NullPolicy.EXCLUDE)])])
