@@ -734,14 +734,32 @@ __global__ void k_nth_element(const __grid_constant__ Channel ch, const uint64_t
 
 // ends[g] = the first (kLast: last) row of group g, among the valid values with
 // skip_nulls; kNoLabel for a group without one.  Rows are taken from that end,
-// so after the first sweep of the grid a row almost never beats the row read
-// and the pass is one read of the labels: 100M rows of 1e4 groups, against
-// 2.2 ms for records of every row sorted by label (which other n still need).
+// so after its first sweep a CTA almost never meets a row that beats the one
+// held, and the pass is one read of the labels.  SMEM: each CTA holds its own
+// ends in shared memory and merges them at the end (read back from L2 for
+// every row, the held rows cost 1,072 us for 100M rows of 1e4 groups; held in
+// shared memory 101 us; records of every row sorted by label, which other n
+// still need, 2.2 ms).
 template <bool kLast>
-__global__ void k_group_end(const __grid_constant__ Channel ch, int64_t n, const uint32_t* __restrict__ labels,
-                            bool skip_nulls, uint32_t* ends, int32_t* status)
+__device__ __forceinline__ void keep_end(uint32_t* p, uint32_t r)
 {
-  constexpr int kRows  = 4;
+  // as a signed maximum the empty marker is -1, below every row
+  if constexpr (kLast) atomicMax(reinterpret_cast<int*>(p), static_cast<int>(r));
+  else atomicMin(p, r);
+}
+
+template <bool kLast, bool SMEM>
+__global__ void __launch_bounds__(SMEM ? 1024 : 256) k_group_end(const __grid_constant__ Channel ch, int64_t n,
+                                                                 const uint32_t* __restrict__ labels, uint32_t G,
+                                                                 bool skip_nulls, uint32_t* ends, int32_t* status)
+{
+  constexpr int kRows = 4;
+  extern __shared__ __align__(16) unsigned char ends_smem[];
+  uint32_t* own = SMEM ? reinterpret_cast<uint32_t*>(ends_smem) : ends;
+  if constexpr (SMEM) {
+    for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) own[g] = kNoLabel;
+    __syncthreads();
+  }
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += kRows * stride) {
     uint32_t label[kRows], held[kRows];
@@ -751,8 +769,11 @@ __global__ void k_group_end(const __grid_constant__ Channel ch, int64_t n, const
       label[q]        = j < n ? __ldg(labels + (kLast ? n - 1 - j : j)) : kNoLabel;
     }
 #pragma unroll
-    for (int q = 0; q < kRows; ++q)
-      held[q] = label[q] != kNoLabel ? Global::ld_u32(reinterpret_cast<uint64_t>(ends + label[q])) : 0u;
+    for (int q = 0; q < kRows; ++q) {
+      held[q] = 0;
+      if (label[q] != kNoLabel)
+        held[q] = SMEM ? own[label[q]] : Global::ld_u32(reinterpret_cast<uint64_t>(own + label[q]));
+    }
 #pragma unroll
     for (int q = 0; q < kRows; ++q) {
       if (label[q] == kNoLabel) continue;
@@ -769,10 +790,13 @@ __global__ void k_group_end(const __grid_constant__ Channel ch, int64_t n, const
           continue;
         }
       }
-      // as a signed maximum the empty marker is -1, below every row
-      if constexpr (kLast) atomicMax(reinterpret_cast<int*>(ends + label[q]), static_cast<int>(r));
-      else atomicMin(ends + label[q], r);
+      keep_end<kLast>(own + label[q], r);
     }
+  }
+  if constexpr (SMEM) {
+    __syncthreads();
+    for (uint32_t g = threadIdx.x; g < G; g += blockDim.x)
+      if (own[g] != kNoLabel) keep_end<kLast>(ends + g, own[g]);
   }
 }
 
@@ -949,9 +973,19 @@ void sorted_kinds(const SortedKindsArgs& a, int* launches)
         // skip a dictionary index is only looked at where it is answered.)
         auto* ends = static_cast<uint32_t*>(sc.get(static_cast<size_t>(G) * 4));
         GBX_CUDA(cudaMemsetAsync(ends, 0xff, static_cast<size_t>(G) * 4, s));
-        const int grid = grid_of(n, a.num_sms);
-        if (o.nth == 0) k_group_end<false><<<grid, 256, 0, s>>>(ch, n, labels, skip, ends, a.status);
-        else k_group_end<true><<<grid, 256, 0, s>>>(ch, n, labels, skip, ends, a.status);
+        // in shared memory up to 48 KB a CTA (two of 1,024 threads an SM, their
+        // merges small beside the rows)
+        const auto g32    = static_cast<uint32_t>(G);
+        const size_t smem = static_cast<size_t>(G) * 4;
+        if (smem <= 48 * 1024 && n >= (int64_t(1) << 20)) {
+          const int grid = 2 * a.num_sms;
+          if (o.nth == 0) k_group_end<false, true><<<grid, 1024, smem, s>>>(ch, n, labels, g32, skip, ends, a.status);
+          else k_group_end<true, true><<<grid, 1024, smem, s>>>(ch, n, labels, g32, skip, ends, a.status);
+        } else {
+          const int grid = grid_of(n, a.num_sms);
+          if (o.nth == 0) k_group_end<false, false><<<grid, 256, 0, s>>>(ch, n, labels, g32, skip, ends, a.status);
+          else k_group_end<true, false><<<grid, 256, 0, s>>>(ch, n, labels, g32, skip, ends, a.status);
+        }
         GBX_CUDA(cudaGetLastError());
         k_row_element<<<grid_of(G, a.num_sms), 256, 0, s>>>(ch, ends, G, o.out_width, o.data, o.mask, o.null_count,
                                                             a.status);
