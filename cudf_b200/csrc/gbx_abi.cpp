@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <string>
@@ -200,6 +201,27 @@ void Alloc::release(void* p, size_t bytes)
   bytes = (bytes + 255) & ~size_t(255);
   if (has_user) user.deallocate(user.ctx, p, bytes, st);
   else cudaFreeAsync(p, st);
+}
+
+void* readback_buffer()
+{
+  struct Buffer {
+    void* p         = nullptr;
+    bool registered = false;
+    ~Buffer()
+    {
+      if (registered) cudaHostUnregister(p);
+      std::free(p);
+    }
+  };
+  thread_local Buffer b;
+  if (b.p == nullptr) {
+    b.p = std::aligned_alloc(kReadbackBytes, kReadbackBytes);
+    if (b.p == nullptr) throw std::bad_alloc();
+    b.registered = cudaHostRegister(b.p, kReadbackBytes, cudaHostRegisterPortable) == cudaSuccess;
+    if (!b.registered) (void)cudaGetLastError();
+  }
+  return b.p;
 }
 
 DeviceInfo current_device()
@@ -918,8 +940,10 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     timer.mark(0);
     // control block: [0..1] sample counters, [2..25] valid counts, [26] status,
     // [27] num_selected, [28..31] partitioned-path counters, [32..33] heavy keys
-    // of the sample and their rows
-    constexpr int kCtlWords = 34;
+    // of the sample and their rows, then the outputs' null counters
+    constexpr int kNullsAt  = 34;
+    constexpr int kCtlWords = kNullsAt + kMaxKeyCols + kMaxOut;
+    static_assert(kCtlWords * 8 <= kReadbackBytes, "the control block fits the read-back buffer");
     auto* ctl = static_cast<unsigned long long*>(scratch.get(kCtlWords * 8));
     GBX_CUDA(cudaMemsetAsync(ctl, 0, kCtlWords * 8, s));
     int32_t* d_status        = reinterpret_cast<int32_t*>(ctl + 26);
@@ -935,16 +959,19 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
 
     // ---- sampled distinct count
     const int64_t nsample = std::min<int64_t>(call.n, 1 << 16);
-    const uint64_t set_cap = 1 << 18;
+    const uint64_t set_cap = next_pow2(4 * static_cast<uint64_t>(nsample));  // 2^18 from 65,536 rows on
     auto* set      = static_cast<uint64_t*>(scratch.get(set_cap * 8));
     auto* set_rows = static_cast<uint32_t*>(scratch.get(set_cap * 4));
     GBX_CUDA(launch_sample(kp_sample, call.n, nsample, set, set_rows, set_cap, ctl, ctl + 32, call.dev.num_sms, s));
     launches += 3;
     timer.mark(1);
 
-    unsigned long long h_ctl[kCtlWords];
-    GBX_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
-    GBX_CUDA(cudaStreamSynchronize(s));
+    auto* const h_ctl = static_cast<unsigned long long*>(readback_buffer());
+    auto read_ctl     = [&]() {
+      GBX_CUDA(cudaMemcpyAsync(h_ctl, ctl, kCtlWords * 8, cudaMemcpyDeviceToHost, s));
+      GBX_CUDA(cudaStreamSynchronize(s));
+    };
+    read_ctl();
     for (size_t i = 0; i < span_owner.size(); ++i) {
       int64_t nulls = static_cast<int64_t>(ms.span[i].size) - static_cast<int64_t>(h_ctl[2 + i]);
       if (span_owner[i].first == 0) key_nulls[span_owner[i].second] = nulls;
@@ -1327,8 +1354,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
           timer.mark(3);
         }
         timer.mark(4);
-        GBX_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
-        GBX_CUDA(cudaStreamSynchronize(s));
+        read_ctl();
         int32_t status;
         std::memcpy(&status, reinterpret_cast<char*>(h_ctl) + 26 * 8, 4);
         Gp = static_cast<int64_t>(h_ctl[30]);
@@ -1382,7 +1408,6 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       for (int a = 0; a < nacc; ++a) t.acc[a] = scratch.get((cap + 1) * acc_bytes(plan.acc.kind[a]));
       t.special_used = reinterpret_cast<uint32_t*>(ctl + 28);
       t.status       = d_status;
-      GBX_CUDA(cudaMemsetAsync(d_status, 0, 4, s));
       GBX_CUDA(launch_init_table(t, plan.acc, plan.key.nwords, call.dev.num_sms, s));
       launches += 1;
       timer.mark(2);
@@ -1436,8 +1461,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       GBX_CUDA(compact_occupied(t, plan.key.nwords, map, d_num_selected, call.dev.num_sms, s));
       launches += 1;
       timer.mark(4);
-      GBX_CUDA(cudaMemcpyAsync(h_ctl, ctl, sizeof(h_ctl), cudaMemcpyDeviceToHost, s));
-      GBX_CUDA(cudaStreamSynchronize(s));
+      read_ctl();
       int32_t status;
       std::memcpy(&status, reinterpret_cast<char*>(h_ctl) + 26 * 8, 4);
       std::memcpy(&G, reinterpret_cast<char*>(h_ctl) + 27 * 8, 8);
@@ -1476,8 +1500,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
 
     // ---- outputs
     OutPlan op     = build_outputs(G);
-    auto* d_nulls  = static_cast<unsigned long long*>(scratch.get((kMaxKeyCols + kMaxOut) * 8));
-    GBX_CUDA(cudaMemsetAsync(d_nulls, 0, (kMaxKeyCols + kMaxOut) * 8, s));
+    auto* d_nulls  = ctl + kNullsAt;  // zeroed with the control block
     op.null_counts = d_nulls;
     GBX_CUDA(launch_finalize(plan, t, map, G, op, call.dev.num_sms, s));
     if (!sorted_outs.empty() && G > 0 && call.n > 0) {
@@ -1518,12 +1541,10 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       gb->stats.kernel_launches += sort_launches;
     }
     timer.mark(5);
-    std::vector<unsigned long long> h_nulls(kMaxKeyCols + kMaxOut, 0);
-    int32_t sort_status = 0;
-    GBX_CUDA(cudaMemcpyAsync(h_nulls.data(), d_nulls, h_nulls.size() * 8, cudaMemcpyDeviceToHost, s));
-    if (!sorted_outs.empty())
-      GBX_CUDA(cudaMemcpyAsync(&sort_status, d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    GBX_CUDA(cudaStreamSynchronize(s));
+    read_ctl();
+    const unsigned long long* h_nulls = h_ctl + kNullsAt;
+    int32_t sort_status               = 0;
+    if (!sorted_outs.empty()) std::memcpy(&sort_status, reinterpret_cast<char*>(h_ctl) + 26 * 8, 4);
     if (sort_status & S_BAD_INDEX) fail(GBX_ERR_LOGIC, "dictionary index out of range");
     if (sort_status & (S_TABLE_FULL | S_SPIN_LIMIT))
       fail(GBX_ERR_DEVICE, "sorted kinds: a row's key was not found in the finished table (status 0x%x)", sort_status);

@@ -100,17 +100,29 @@ struct Alloc {
   void release(void* p, size_t bytes);
 };
 
-// Scratch buffers released (stream-ordered) when the owner goes away.
+// Scratch buffers released (stream-ordered) when the owner goes away.  Small
+// buffers are carved from shared blocks of kBlock bytes: a call takes a dozen
+// of them, and a caller's allocator costs microseconds each (a 10K-row call
+// spends most of its time on the host).
 struct Scratch {
+  static constexpr size_t kBlock = size_t(4) << 20;
   Alloc* a;
   std::vector<std::pair<void*, size_t>> bufs;
+  unsigned char* block = nullptr;  // the block being carved
+  size_t used          = 0;
   explicit Scratch(Alloc* al) : a(al) {}
   Scratch(const Scratch&)            = delete;
   Scratch& operator=(const Scratch&) = delete;
   void* get(size_t bytes)
   {
-    void* p = a->allocate(bytes);
-    bufs.emplace_back(p, bytes);
+    const size_t need = ((bytes == 0 ? 8 : bytes) + 255) & ~size_t(255);
+    if (need > kBlock / 2) return own(bytes);
+    if (block == nullptr || used + need > kBlock) {
+      block = static_cast<unsigned char*>(own(kBlock));
+      used  = 0;
+    }
+    void* p = block + used;
+    used += need;
     return p;
   }
   size_t total() const
@@ -123,9 +135,28 @@ struct Scratch {
   {
     for (auto& b : bufs) a->release(b.first, b.second);
     bufs.clear();
+    block = nullptr;
+    used  = 0;
   }
   ~Scratch() { release_all(); }
+
+ private:
+  void* own(size_t bytes)
+  {
+    void* p = a->allocate(bytes);
+    bufs.emplace_back(p, bytes);
+    return p;
+  }
 };
+
+// A page-locked host buffer of this thread for the small results a call reads
+// back (a copy to pageable memory is staged by the driver and costs several
+// microseconds more).  Every use is synchronised before the next, so one
+// buffer per thread serves any stream.  It is ordinary memory registered with
+// the driver: where that fails, or a device reset has undone it, the copies
+// are staged as before.  Given back when the thread ends.
+constexpr size_t kReadbackBytes = 4096;
+void* readback_buffer();
 
 struct DeviceInfo {
   int device        = -1;

@@ -179,12 +179,21 @@ __global__ void k_sample_heavy(const uint32_t* set_rows, uint64_t set_cap, unsig
   }
 }
 
-__global__ void k_fill_u64(uint64_t* p, uint64_t n, uint64_t v)
+// Empties the sample's set, its row counts and the counters of both.
+__global__ void k_clear_sample(uint64_t* set, uint32_t* rows, uint64_t n, unsigned long long* counters,
+                               unsigned long long* heavy)
 {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
+  const uint64_t i0     = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (uint64_t i = i0; i < n; i += stride) {
+    set[i]  = kEmptyWord;
+    rows[i] = 0;
+  }
+  if (i0 < 2) {
+    counters[i0] = 0;
+    heavy[i0]    = 0;
+  }
 }
-
 
 // ------------------------------------------------------------- finalize
 
@@ -381,11 +390,7 @@ cudaError_t launch_sample(const KeyPlan& kp, int64_t n, int64_t nsample, uint64_
                           cudaStream_t st)
 {
   const int fill_grid = grid_for(static_cast<int64_t>(set_cap), 256, num_sms * 8);
-  k_fill_u64<<<fill_grid, 256, 0, st>>>(set, set_cap, kEmptyWord);
-  cudaError_t e = cudaMemsetAsync(set_rows, 0, set_cap * sizeof(uint32_t), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(heavy, 0, 2 * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
+  k_clear_sample<<<fill_grid, 256, 0, st>>>(set, set_rows, set_cap, counters, heavy);
   int grid = grid_for(nsample, 256, num_sms * 8);
   if (kp.nwords == 1) k_sample_distinct<1><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
   else k_sample_distinct<2><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
