@@ -42,6 +42,7 @@ constexpr int kJPer              = 8;  // probe rows of a thread
 constexpr int kJFlight           = 4;  // of which so many probe at a time
 constexpr int kJTile             = kJBlock * kJPer;
 constexpr uint32_t kNoSlot       = 0xffffffffu;
+constexpr uintptr_t kSectorBytes = 32;  // a load_sector, aligned
 // build rows up to which a slot index (the reserved slot included) stays
 // below kNoSlot
 constexpr int64_t kMaxBuildRows = int64_t(1) << 30;
@@ -470,7 +471,9 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   const size_t nb4 = static_cast<size_t>(nb) * 4;
   PackedTable t{};
   t.cap         = cap;
-  t.slots       = static_cast<Slot*>(sc.get((cap + 1) * sizeof(Slot)));
+  // 32-byte sectors, whatever the caller's allocator aligns to
+  const auto raw = reinterpret_cast<uintptr_t>(sc.get((cap + 1) * sizeof(Slot) + kSectorBytes - 1));
+  t.slots        = reinterpret_cast<Slot*>((raw + kSectorBytes - 1) & ~(kSectorBytes - 1));
   auto* flags   = static_cast<uint32_t*>(sc.get(8));  // repeated keys, cursor of the ranges
   t.dup         = flags;
   auto* slot_of = static_cast<uint32_t*>(sc.get(nb4));

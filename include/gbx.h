@@ -187,7 +187,9 @@ typedef struct gbx_request {
 } gbx_request;
 
 /* Stream-ordered device allocator (rmm::device_async_resource_ref).
- * `stream` is a cudaStream_t.  Pass NULL to use cudaMallocAsync/cudaFreeAsync. */
+ * `stream` is a cudaStream_t.  Memory must be aligned to 16 bytes at least
+ * (128-bit atomics and 16-byte copies run on it).  Pass NULL to use
+ * cudaMallocAsync/cudaFreeAsync. */
 typedef struct gbx_allocator {
   void* ctx;
   void* (*allocate)(void* ctx, size_t bytes, void* stream);
