@@ -37,3 +37,17 @@ def test_two_word_keys():
     keys = [HostCol(rng.integers(-2, 40, n).astype(np.int64)), HostCol(rng.integers(-1, 9, n).astype(np.int64))]
     T.assert_parity(keys, [(HostCol(rng.integers(0, 99, n).astype(np.int16)),
                             [_nth(0, NullPolicy.INCLUDE), _nth(-1, NullPolicy.EXCLUDE)])])
+
+
+@pytest.mark.parametrize("n,groups", [(1600, 899), (1600, 900), (1600, 901), (70_000, 39_374),
+                                      (70_000, 39_376), (5000, 5000)])
+def test_few_rows_a_group(n, groups):
+    """Both sides of the line between the label table and the global table (16 groups to 9 rows)."""
+    rng = np.random.default_rng(n + groups)
+    k = np.concatenate([np.arange(groups), rng.integers(0, groups, n - groups)])
+    k = rng.permutation(k).astype(np.int64) * 31 - 31
+    k[k == -31] = -1  # the all-ones word
+    v = rng.integers(-1000, 1000, n).astype(np.int64)
+    T.assert_parity([HostCol(k, rng.random(n) >= 0.01 if groups % 2 else None)],
+                    [(HostCol(v), [(Kind.MEDIAN, 0), (Kind.NUNIQUE, 0, {"null_policy": NullPolicy.EXCLUDE}),
+                                   _nth(0, NullPolicy.INCLUDE), _nth(1, NullPolicy.EXCLUDE)])])
