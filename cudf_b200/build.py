@@ -87,3 +87,20 @@ def build_facade_test(verbose: bool = False) -> str:
         print(" ".join(cmd), file=sys.stderr)
     subprocess.run(cmd, check=True)
     return FACADE_TEST_BIN
+
+
+LABELS_TEST_SRC = os.path.join(os.path.dirname(HERE), "tests", "cpp", "sorted_labels_test.cu")
+LABELS_TEST_BIN = os.path.join(os.path.dirname(HERE), "tests", "cpp", "_build", "sorted_labels_test")
+
+
+def build_labels_test(verbose: bool = False) -> str:
+    """Compiles the test of the sorted kinds' labels against the library's own objects."""
+    build_library()
+    os.makedirs(os.path.dirname(LABELS_TEST_BIN), exist_ok=True)
+    objs = [os.path.join(CSRC, "_build", src + ".o") for src in SOURCES]
+    cmd = [nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O2", LABELS_TEST_SRC,
+           *objs, "-o", LABELS_TEST_BIN]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    subprocess.run(cmd, check=True)
+    return LABELS_TEST_BIN

@@ -152,9 +152,10 @@ __device__ __forceinline__ uint32_t label_hash(uint64_t k)
   return tile_hash<1>(one);
 }
 
-// Enters the G occupied slots `map` of the global table.
+// Enters the G occupied slots `map` of the global table (a key without room:
+// S_TABLE_FULL).
 __global__ void k_label_table(const __grid_constant__ TableRef t, const uint32_t* __restrict__ map, int64_t G,
-                              const LabelTable lt)
+                              const LabelTable lt, int32_t* status)
 {
   for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < G;
        g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -165,7 +166,8 @@ __global__ void k_label_table(const __grid_constant__ TableRef t, const uint32_t
     }
     const uint64_t k = t.keys[slot];
     uint32_t s       = label_hash(k) & (lt.slots - 1);
-    for (uint32_t p = 0; p < lt.slots; ++p) {  // distinct keys, fewer than slots: an empty one is met
+    uint32_t p       = 0;
+    for (; p < lt.slots; ++p) {  // distinct keys, fewer than slots: an empty one is met
       if (atomicCAS(reinterpret_cast<unsigned long long*>(lt.keys + s), static_cast<unsigned long long>(kEmptyWord),
                     static_cast<unsigned long long>(k)) == kEmptyWord) {
         lt.rows[s] = static_cast<uint32_t>(g);
@@ -173,13 +175,15 @@ __global__ void k_label_table(const __grid_constant__ TableRef t, const uint32_t
       }
       s = (s + 1) & (lt.slots - 1);
     }
+    if (p == lt.slots) atomicOr(status, S_TABLE_FULL);
   }
 }
 
 constexpr int kLabelPer = 4;  // rows a thread probes together
 
 // labels[r] = the output row of row r's group (kNoLabel for a row whose key
-// is excluded), one-word keys.  SMEM: every CTA copies the label table into
+// is excluded; a kept key that is not found sets S_TABLE_FULL, as the probe of
+// the global table does), one-word keys.  SMEM: every CTA copies the label table into
 // shared memory (label rows as 16 bits) and probes it there; otherwise it is
 // read through L1.  The probe of the global table this replaces bypassed L1
 // with one row a thread: 2,798 us for 100M rows of 1e4 groups, bound by the
@@ -187,7 +191,8 @@ constexpr int kLabelPer = 4;  // rows a thread probes together
 template <bool SMEM>
 __global__ void __launch_bounds__(SMEM ? 1024 : 256) k_row_labels_one(const __grid_constant__ Plan plan, int64_t n,
                                                                       const LabelTable lt,
-                                                                      uint32_t* __restrict__ labels)
+                                                                      uint32_t* __restrict__ labels,
+                                                                      int32_t* status)
 {
   extern __shared__ __align__(16) unsigned char label_smem[];
   uint64_t* skeys = reinterpret_cast<uint64_t*>(label_smem);
@@ -242,9 +247,13 @@ __global__ void __launch_bounds__(SMEM ? 1024 : 256) k_row_labels_one(const __gr
       }
     }
     __syncwarp();
+    bool missed = false;
 #pragma unroll
-    for (int q = 0; q < kLabelPer; ++q)
+    for (int q = 0; q < kLabelPer; ++q) {
       if ((in >> q) & 1u) labels[r0 + q * step] = label[q];
+      missed = missed || (((kept >> q) & 1u) && label[q] == kNoLabel);
+    }
+    if (missed) atomicOr(status, S_TABLE_FULL);
   }
 }
 
@@ -874,7 +883,7 @@ void sorted_kinds(const SortedKindsArgs& a, int* launches)
     lt.special = static_cast<uint32_t*>(sc.get(8));
     GBX_CUDA(cudaMemsetAsync(lt.keys, 0xff, static_cast<size_t>(lt.slots) * 8, s));
     GBX_CUDA(cudaMemsetAsync(lt.special, 0xff, 8, s));
-    k_label_table<<<grid_of(G, a.num_sms), 256, 0, s>>>(a.table, a.map, G, lt);
+    k_label_table<<<grid_of(G, a.num_sms), 256, 0, s>>>(a.table, a.map, G, lt, a.status);
     GBX_CUDA(cudaGetLastError());
     // up to 16,384 slots (160 KB, 12,288 groups) the table fits shared memory;
     // few rows do not pay for the copies
@@ -882,9 +891,10 @@ void sorted_kinds(const SortedKindsArgs& a, int* launches)
     if (lt.slots <= 16384 && n >= (int64_t(1) << 20)) {
       GBX_CUDA(ensure_dynamic_smem(reinterpret_cast<const void*>(k_row_labels_one<true>), smem));
       const int ctas = smem <= 100 * 1024 ? 2 : 1;
-      k_row_labels_one<true><<<a.num_sms * ctas, 1024, smem, s>>>(a.plan, n, lt, labels);
+      k_row_labels_one<true><<<a.num_sms * ctas, 1024, smem, s>>>(a.plan, n, lt, labels, a.status);
     } else {
-      k_row_labels_one<false><<<grid_of((n + kLabelPer - 1) / kLabelPer, a.num_sms), 256, 0, s>>>(a.plan, n, lt, labels);
+      k_row_labels_one<false>
+        <<<grid_of((n + kLabelPer - 1) / kLabelPer, a.num_sms), 256, 0, s>>>(a.plan, n, lt, labels, a.status);
     }
   } else {
     auto* inv = static_cast<uint32_t*>(sc.get((a.table.cap + 1) * sizeof(uint32_t)));

@@ -4,9 +4,13 @@ the all-ones key, two-word keys, excluded keys, and n = 0 / -1 under both null
 policies beside another n."""
 from __future__ import annotations
 
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
+from cudf_b200 import build
 from cudf_b200._abi import Kind, NullPolicy
 from oracle.oracle import HostCol
 from tests import gbx_testing as T
@@ -51,3 +55,12 @@ def test_few_rows_a_group(n, groups):
     T.assert_parity([HostCol(k, rng.random(n) >= 0.01 if groups % 2 else None)],
                     [(HostCol(v), [(Kind.MEDIAN, 0), (Kind.NUNIQUE, 0, {"null_policy": NullPolicy.EXCLUDE}),
                                    _nth(0, NullPolicy.INCLUDE), _nth(1, NullPolicy.EXCLUDE)])])
+
+
+def test_a_key_missing_from_the_table_is_reported():
+    """sorted_kinds() on a hand-made table (tests/cpp/sorted_labels_test.cu)."""
+    exe = build.LABELS_TEST_BIN
+    if not os.path.exists(exe) or os.path.getmtime(exe) < max(map(os.path.getmtime, (build.LABELS_TEST_SRC, build.LIB))):
+        build.build_labels_test()
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "0 failure(s)" in r.stdout, r.stdout + r.stderr
