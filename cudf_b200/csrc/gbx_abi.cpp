@@ -944,6 +944,9 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     constexpr int kNullsAt  = 34;
     constexpr int kCtlWords = kNullsAt + kMaxKeyCols + kMaxOut;
     static_assert(kCtlWords * 8 <= kReadbackBytes, "the control block fits the read-back buffer");
+    const int64_t nsample  = std::min<int64_t>(call.n, 1 << 16);
+    const uint64_t set_cap = next_pow2(4 * static_cast<uint64_t>(nsample));  // 2^18 from 65,536 rows on
+    scratch.together({kCtlWords * 8, set_cap * 8, set_cap * 4});
     auto* ctl = static_cast<unsigned long long*>(scratch.get(kCtlWords * 8));
     GBX_CUDA(cudaMemsetAsync(ctl, 0, kCtlWords * 8, s));
     int32_t* d_status        = reinterpret_cast<int32_t*>(ctl + 26);
@@ -958,8 +961,6 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       fail(GBX_ERR_UNSUPPORTED, "key columns need more than 128 packed bits; wider composite keys are not supported");
 
     // ---- sampled distinct count
-    const int64_t nsample = std::min<int64_t>(call.n, 1 << 16);
-    const uint64_t set_cap = next_pow2(4 * static_cast<uint64_t>(nsample));  // 2^18 from 65,536 rows on
     auto* set      = static_cast<uint64_t*>(scratch.get(set_cap * 8));
     auto* set_rows = static_cast<uint32_t*>(scratch.get(set_cap * 4));
     GBX_CUDA(launch_sample(kp_sample, call.n, nsample, set, set_rows, set_cap, ctl, ctl + 32, call.dev.num_sms, s));
@@ -1264,6 +1265,8 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
         pp.status       = d_status;
         auto arr        = [&]() { return static_cast<uint32_t*>(scratch.get((static_cast<size_t>(P) + 1) * 4)); };
         const size_t nctr = (static_cast<size_t>(P) << pp.shard_bits) + 1;
+        const size_t p4   = (static_cast<size_t>(P) + 1) * 4;
+        scratch.together({nctr * 4, nctr * 4, nctr * 4, p4, p4, p4, p4});
         pp.counts       = static_cast<uint32_t*>(scratch.get(nctr * 4));
         pp.offsets      = static_cast<uint32_t*>(scratch.get(nctr * 4));
         pp.cursor       = static_cast<uint32_t*>(scratch.get(nctr * 4));
@@ -1403,9 +1406,13 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       // ---- table
       t     = TableRef{};
       t.cap = cap;
+      std::vector<size_t> sizes{(cap + 1) * plan.key.nwords * 8, (cap + 1) * 4, (cap + 1) * 4};
+      for (int a = 0; a < nacc; ++a) sizes.push_back((cap + 1) * acc_bytes(plan.acc.kind[a]));
+      scratch.together(sizes);
       t.keys = static_cast<uint64_t*>(scratch.get((cap + 1) * plan.key.nwords * 8));
       t.rows = static_cast<uint32_t*>(scratch.get((cap + 1) * 4));
       for (int a = 0; a < nacc; ++a) t.acc[a] = scratch.get((cap + 1) * acc_bytes(plan.acc.kind[a]));
+      map            = static_cast<uint32_t*>(scratch.get((cap + 1) * 4));
       t.special_used = reinterpret_cast<uint32_t*>(ctl + 28);
       t.status       = d_status;
       GBX_CUDA(launch_init_table(t, plan.acc, plan.key.nwords, call.dev.num_sms, s));
@@ -1443,6 +1450,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
         auto* roffsets     = static_cast<uint32_t*>(scratch.get(part_radix_count_bytes(call.n)));
         size_t rtemp_bytes = 0;
         GBX_CUDA(part_radix_temp_bytes(call.n, &rtemp_bytes));
+        scratch.together({rtemp_bytes, sizeof(uint32_t)});
         void* rtemp  = scratch.get(rtemp_bytes);
         auto* n_kept = static_cast<uint32_t*>(scratch.get(sizeof(uint32_t)));
         GBX_CUDA(launch_part_radix_hist0(plan, call.n, bucket_bits, rcounts, nullptr, s));
@@ -1457,7 +1465,6 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       launches += 1;
       timer.mark(3);
       // ---- compaction of occupied slots
-      map = static_cast<uint32_t*>(scratch.get((cap + 1) * 4));
       GBX_CUDA(compact_occupied(t, plan.key.nwords, map, d_num_selected, call.dev.num_sms, s));
       launches += 1;
       timer.mark(4);

@@ -496,6 +496,7 @@ int gbx_distinct_join(const gbx_table_view* build, const gbx_table_view* probe, 
     const uint64_t cap = next_pow2(std::max<uint64_t>(2 * static_cast<uint64_t>(nb) + 2, 64));
     TableRef t{};
     t.cap          = cap;
+    sc.together({(cap + 1) * NW * 8, 8, 8, (cap + 1) * 4, 8});
     t.keys         = static_cast<uint64_t*>(sc.get((cap + 1) * NW * 8));
     t.special_used = static_cast<uint32_t*>(sc.get(8));
     t.status       = static_cast<int32_t*>(sc.get(8));

@@ -100,30 +100,43 @@ struct Alloc {
   void release(void* p, size_t bytes);
 };
 
-// Scratch buffers released (stream-ordered) when the owner goes away.  Small
-// buffers are carved from shared blocks of kBlock bytes: a call takes a dozen
-// of them, and a caller's allocator costs microseconds each (a 10K-row call
-// spends most of its time on the host).
+// Scratch buffers released (stream-ordered) when the owner goes away.  A call
+// takes a dozen small ones, and a caller's allocator costs microseconds each
+// (a 10K-row call spends most of its time on the host), so sizes known
+// together() share one allocation of exactly their sum: fewer allocations,
+// and no more memory than one each.
 struct Scratch {
-  static constexpr size_t kBlock = size_t(4) << 20;
+  static constexpr size_t kSmall = size_t(2) << 20;  // a buffer beyond this is allocated by itself
   Alloc* a;
   std::vector<std::pair<void*, size_t>> bufs;
-  unsigned char* block = nullptr;  // the block being carved
+  unsigned char* block = nullptr;  // the allocation being carved
   size_t used          = 0;
+  size_t block_bytes   = 0;
   explicit Scratch(Alloc* al) : a(al) {}
   Scratch(const Scratch&)            = delete;
   Scratch& operator=(const Scratch&) = delete;
   void* get(size_t bytes)
   {
-    const size_t need = ((bytes == 0 ? 8 : bytes) + 255) & ~size_t(255);
-    if (need > kBlock / 2) return own(bytes);
-    if (block == nullptr || used + need > kBlock) {
-      block = static_cast<unsigned char*>(own(kBlock));
-      used  = 0;
-    }
+    const size_t need = rounded(bytes);
+    if (need > kSmall || used + need > block_bytes) return own(bytes);
     void* p = block + used;
     used += need;
     return p;
+  }
+  // The get() calls that follow ask for these sizes.
+  void together(const std::vector<size_t>& sizes)
+  {
+    size_t sum = 0;
+    for (size_t b : sizes) sum += rounded(b) <= kSmall ? rounded(b) : 0;
+    block = nullptr;
+    used = block_bytes = 0;
+    if (sum == 0) return;
+    try {
+      block       = static_cast<unsigned char*>(own(sum));
+      block_bytes = sum;
+    } catch (const Failure&) {
+      // no room for them in one piece: one by one
+    }
   }
   size_t total() const
   {
@@ -136,11 +149,12 @@ struct Scratch {
     for (auto& b : bufs) a->release(b.first, b.second);
     bufs.clear();
     block = nullptr;
-    used  = 0;
+    used = block_bytes = 0;
   }
   ~Scratch() { release_all(); }
 
  private:
+  static size_t rounded(size_t bytes) { return ((bytes == 0 ? 8 : bytes) + 255) & ~size_t(255); }
   void* own(size_t bytes)
   {
     void* p = a->allocate(bytes);

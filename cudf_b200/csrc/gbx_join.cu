@@ -261,6 +261,7 @@ int64_t distinct_by_representatives(const gbx_table_view* keys, int32_t keep, in
   Scratch sc(&a);
   const size_t n4    = static_cast<size_t>(n) * 4;
   const uint64_t cap = next_pow2(std::max<uint64_t>(2 * static_cast<uint64_t>(n) + 2, 64));
+  sc.together({cap * 4, n4, n4, n4, n4, n4, n4, 8});
   auto* slots  = static_cast<int32_t*>(sc.get(cap * 4));
   auto* rep    = static_cast<int32_t*>(sc.get(n4));
   auto* fmin   = static_cast<int32_t*>(sc.get(n4));
@@ -353,6 +354,7 @@ int gbx_hash_join(const gbx_table_view* left, const gbx_table_view* right, int32
     const size_t nb4 = static_cast<size_t>(std::max<int64_t>(nb, 1)) * 4;
     const size_t np4 = static_cast<size_t>(std::max<int64_t>(np, 1)) * 4;
     const uint64_t cap = next_pow2(std::max<uint64_t>(2 * static_cast<uint64_t>(nb) + 2, 64));
+    sc.together({cap * 4, nb4, nb4, nb4, nb4, nb4, np4, np4 * 2, np4 * 2, 8});
     auto* slots  = static_cast<int32_t*>(sc.get(cap * 4));
     auto* rep    = static_cast<int32_t*>(sc.get(nb4));
     auto* cnt    = static_cast<uint32_t*>(sc.get(nb4));

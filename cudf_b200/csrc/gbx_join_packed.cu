@@ -471,21 +471,25 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   const size_t nb4 = static_cast<size_t>(nb) * 4;
   PackedTable t{};
   t.cap         = cap;
+  const size_t slot_bytes = (cap + 1) * sizeof(Slot) + kSectorBytes - 1;
+  const size_t np4        = static_cast<size_t>(np) * 4;
+  const size_t tile_bytes = static_cast<size_t>(ntiles + 1) * 8;
+  size_t tb32 = 0, tb64 = 0;
+  GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, nb, nullptr, &tb32, s));
+  GBX_CUDA(scan_exclusive_i64(nullptr, nullptr, ntiles + 1, nullptr, &tb64, s));
+  size_t tbytes = std::max(std::max(tb32, tb64), size_t(1));
+  sc.together({slot_bytes, 8, nb4, nb4, nb4, np4, tile_bytes, tbytes});
   // 32-byte sectors, whatever the caller's allocator aligns to
-  const auto raw = reinterpret_cast<uintptr_t>(sc.get((cap + 1) * sizeof(Slot) + kSectorBytes - 1));
+  const auto raw = reinterpret_cast<uintptr_t>(sc.get(slot_bytes));
   t.slots        = reinterpret_cast<Slot*>((raw + kSectorBytes - 1) & ~(kSectorBytes - 1));
   auto* flags   = static_cast<uint32_t*>(sc.get(8));  // repeated keys, cursor of the ranges
   t.dup         = flags;
   auto* slot_of = static_cast<uint32_t*>(sc.get(nb4));
   auto* rank_of = static_cast<uint32_t*>(sc.get(nb4));
   auto* rows    = static_cast<int32_t*>(sc.get(nb4));
-  auto* match   = static_cast<uint32_t*>(sc.get(static_cast<size_t>(np) * 4));
-  auto* tiles   = static_cast<int64_t*>(sc.get(static_cast<size_t>(ntiles + 1) * 8));
-  size_t tb32 = 0, tb64 = 0;
-  GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, nb, nullptr, &tb32, s));
-  GBX_CUDA(scan_exclusive_i64(nullptr, nullptr, ntiles + 1, nullptr, &tb64, s));
-  size_t tbytes = std::max(tb32, tb64);
-  void* temp    = sc.get(std::max<size_t>(tbytes, 1));
+  auto* match   = static_cast<uint32_t*>(sc.get(np4));
+  auto* tiles   = static_cast<int64_t*>(sc.get(tile_bytes));
+  void* temp    = sc.get(tbytes);
 
   // 1. the table
   GBX_CUDA(cudaMemsetAsync(flags, 0, 8, s));

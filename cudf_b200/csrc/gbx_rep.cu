@@ -456,10 +456,13 @@ int aggregate_by_representatives(gbx_groupby* gb, const std::vector<gbx_column_v
   const KeyTree tree = key_tree(keys, null_policy);
   const RepKeys& rk   = tree.rk;
   const uint64_t cap = next_pow2(std::max<uint64_t>(2 * static_cast<uint64_t>(n) + 2, 64));
+  const size_t n4   = static_cast<size_t>(std::max<int64_t>(n, 1)) * 4;
+  const size_t bits = static_cast<size_t>((n + 31) / 32) * 4 + 64;
+  sc.together({cap * 4, n4, 8, bits});
   auto* slots  = static_cast<int32_t*>(sc.get(cap * 4));
-  auto* rep    = static_cast<int32_t*>(sc.get(static_cast<size_t>(std::max<int64_t>(n, 1)) * 4));
+  auto* rep    = static_cast<int32_t*>(sc.get(n4));
   auto* status = static_cast<int32_t*>(sc.get(8));
-  auto* mask   = static_cast<uint32_t*>(sc.get(static_cast<size_t>((n + 31) / 32) * 4 + 64));
+  auto* mask   = static_cast<uint32_t*>(sc.get(bits));
   GBX_CUDA(cudaMemsetAsync(status, 0, 8, s));
   k_fill_i32<<<grid_of(static_cast<int64_t>(cap), num_sms), kRepBlock, 0, s>>>(slots, -1, static_cast<int64_t>(cap));
   GBX_CUDA(cudaGetLastError());
@@ -530,6 +533,7 @@ int aggregate_presorted(gbx_groupby* gb, const std::vector<gbx_column_view>& key
   const bool by_key = rk.exclude_nulls && null_keys;
 
   const size_t nb = static_cast<size_t>(std::max<int64_t>(n, 1)) * 4;
+  sc.together({nb, nb, nb, nb, 8});
   auto* label     = static_cast<int32_t*>(sc.get(nb));
   auto* first     = static_cast<int32_t*>(sc.get(nb));
   auto* flags     = static_cast<uint32_t*>(sc.get(nb));
@@ -673,10 +677,12 @@ int aggregate_string_extrema(gbx_groupby* gb, const std::vector<gbx_column_view>
   const KeyTree tree = key_tree(keys, null_policy);
   const RepKeys& rk  = tree.rk;
   const uint64_t cap = next_pow2(std::max<uint64_t>(2 * static_cast<uint64_t>(n) + 2, 64));
+  const size_t bits = static_cast<size_t>((n + 31) / 32) * 4 + 64;
+  sc.together({cap * 4, n4, 8, bits});
   auto* slots  = static_cast<int32_t*>(sc.get(cap * 4));
   auto* rep    = static_cast<int32_t*>(sc.get(n4));
   auto* status = static_cast<int32_t*>(sc.get(8));
-  auto* mask   = static_cast<uint32_t*>(sc.get(static_cast<size_t>((n + 31) / 32) * 4 + 64));
+  auto* mask   = static_cast<uint32_t*>(sc.get(bits));
   GBX_CUDA(cudaMemsetAsync(status, 0, 8, s));
   k_fill_i32<<<grid_of(static_cast<int64_t>(cap), num_sms), kRepBlock, 0, s>>>(slots, -1, static_cast<int64_t>(cap));
   GBX_CUDA(cudaGetLastError());

@@ -878,6 +878,7 @@ void sorted_kinds(const SortedKindsArgs& a, int* launches)
   if (a.plan.key.nwords == 1 && 16 * G <= 9 * n) {
     LabelTable lt{};
     lt.slots = static_cast<uint32_t>(next_pow2(std::max<uint64_t>(static_cast<uint64_t>(G) * 4 / 3 + 1, 64)));
+    sc.together({static_cast<size_t>(lt.slots) * 8, static_cast<size_t>(lt.slots) * 4, 8});
     lt.keys  = static_cast<uint64_t*>(sc.get(static_cast<size_t>(lt.slots) * 8));
     lt.rows  = static_cast<uint32_t*>(sc.get(static_cast<size_t>(lt.slots) * 4));
     lt.special = static_cast<uint32_t*>(sc.get(8));
@@ -911,17 +912,19 @@ void sorted_kinds(const SortedKindsArgs& a, int* launches)
   // ping-pong copies, tile counts, scan scratch
   const int ntiles    = static_cast<int>((n + kSortTile - 1) / kSortTile);
   const size_t nrec   = static_cast<size_t>(n);
-  auto* lo0           = static_cast<uint64_t*>(sc.get(nrec * 8));
-  auto* lo1           = static_cast<uint64_t*>(sc.get(nrec * 8));
-  uint32_t* hi0       = nullptr;
-  uint32_t* hi1       = nullptr;
   const int64_t items = static_cast<int64_t>(ntiles) * 256;
-  auto* counts        = static_cast<uint32_t*>(sc.get(static_cast<size_t>(items) * 4));
-  auto* offsets       = static_cast<uint32_t*>(sc.get(static_cast<size_t>(items) * 4));
   size_t tb_items = 0, tb_flags = 0;
   GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, items, nullptr, &tb_items, s));
   GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, n + 1, nullptr, &tb_flags, s));
   const size_t tb = std::max(tb_items, tb_flags);
+  sc.together({nrec * 8, nrec * 8, static_cast<size_t>(items) * 4, static_cast<size_t>(items) * 4, tb,
+               static_cast<size_t>(G) * 3 * sizeof(int64_t), sizeof(Range)});
+  auto* lo0       = static_cast<uint64_t*>(sc.get(nrec * 8));
+  auto* lo1       = static_cast<uint64_t*>(sc.get(nrec * 8));
+  uint32_t* hi0   = nullptr;
+  uint32_t* hi1   = nullptr;
+  auto* counts    = static_cast<uint32_t*>(sc.get(static_cast<size_t>(items) * 4));
+  auto* offsets   = static_cast<uint32_t*>(sc.get(static_cast<size_t>(items) * 4));
   void* temp      = sc.get(tb);
   auto* bounds    = static_cast<int64_t*>(sc.get(static_cast<size_t>(G) * 3 * sizeof(int64_t)));
   auto* range     = static_cast<Range*>(sc.get(sizeof(Range)));

@@ -1,11 +1,13 @@
 """Calls through a caller's own gbx_allocator: memory aligned to 16 bytes only
-(what the interface asks for).  Results against numpy, bit for bit."""
+(what the interface asks for), and pools with little room.  Results against
+numpy, bit for bit."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
-from cudf_b200 import Table
+from cudf_b200 import Column, GroupBy, GroupByRequest, Table
+from cudf_b200 import aggregation as agg
 from cudf_b200 import join as J
 from cudf_b200.groupby import TorchAllocator
 from oracle.oracle import HostCol
@@ -30,6 +32,31 @@ class OffsetAllocator(TorchAllocator):
         return p + self.offset
 
 
+class TightAllocator(TorchAllocator):
+    """Refuses a request beyond `largest` bytes, or one that takes the live bytes beyond `room`."""
+
+    def __init__(self, largest, room=1 << 62):
+        super().__init__()
+        self.largest, self.room = largest, room
+
+    def _allocate(self, ctx, nbytes, stream):
+        if int(nbytes) > self.largest or self.current + int(nbytes) > self.room:
+            return None
+        return super()._allocate(ctx, nbytes, stream)
+
+
+def _sums(keys, allocator):
+    """{key: rows} of a groupby over the key column, through the allocator."""
+    n = len(keys)
+    column = Column.from_strings(keys) if isinstance(keys, list) else T.device_column(HostCol(keys))
+    gk, res = GroupBy(Table([column])).aggregate(
+        [GroupByRequest(T.device_column(HostCol(np.ones(n, dtype=np.int64))), [agg.sum(), agg.median()])],
+        allocator=allocator)
+    cols = res[0].columns()
+    assert np.all(cols[1].to_numpy()[0] == 1.0)
+    return dict(zip(gk.columns()[0].to_numpy()[0].tolist(), cols[0].to_numpy()[0].tolist()))
+
+
 def _pairs(cols):
     return sorted(zip(*(c.to_numpy()[0].tolist() for c in cols)))
 
@@ -43,3 +70,30 @@ def test_packed_join_on_memory_aligned_to_16_bytes(rows, offset):
                         Table([T.device_column(HostCol(right.astype(np.int64)))]), allocator=OffsetAllocator(offset))
     where = {int(k): i for i, k in enumerate(right)}
     assert _pairs(cols) == [(i, where[int(k)]) for i, k in enumerate(left) if int(k) in where]
+
+
+@pytest.mark.parametrize("strings", [False, True], ids=["int64", "string"])
+def test_a_small_call_asks_for_little(strings):
+    """A 100-row call takes kilobytes (a table of 1,024 slots is the most of it), not a block of megabytes."""
+    k = np.arange(100, dtype=np.int64) % 7
+    want = {int(i): int((k == i).sum()) for i in range(7)}
+    if strings:
+        k = [f"key {i}" for i in k]
+        want = {f"key {i}": n for i, n in want.items()}
+    pool = TightAllocator(256 << 10, 512 << 10)
+    assert _sums(k, pool) == want
+    assert pool.peak <= 256 << 10
+
+
+def test_a_small_join_asks_for_little():
+    left, right = np.arange(100, dtype=np.int64), np.arange(50, dtype=np.int64)
+    pool = TightAllocator(64 << 10)
+    got = J.inner_join(Table([T.device_column(HostCol(left))]), Table([T.device_column(HostCol(right))]), allocator=pool)
+    assert _pairs(got) == [(i, i) for i in range(50)]
+    assert pool.peak <= 64 << 10
+
+
+def test_buffers_that_do_not_fit_in_one_piece_come_one_by_one():
+    """20,000 rows: the sample's buffers together are 1.5 MB, the largest of them 1 MB."""
+    k = np.arange(20_000, dtype=np.int64) % 100
+    assert _sums(k, TightAllocator(1 << 20)) == {i: 200 for i in range(100)}
