@@ -336,10 +336,20 @@ int gbx_hash_join(const gbx_table_view* left, const gbx_table_view* right, int32
     const gbx_table_view* probe = swap ? right : left;
     const int64_t nb = build->columns[0].size;
     const int64_t np = probe->columns[0].size;
-    // keys of one packed word carry the key in the slot (gbx_join_packed.cu)
-    if (packed_join(build, probe, compare_nulls, join_kind, a, swap ? *right_indices : *left_indices,
-                    swap ? *left_indices : *right_indices))
-      return;
+    gbx_column& out_probe = swap ? *right_indices : *left_indices;
+    gbx_column& out_build = swap ? *left_indices : *right_indices;
+    // keys of one packed word carry the key in the slot (gbx_join_packed.cu);
+    // its table takes 21 to 43 bytes a build row where the one below takes 8
+    // to 16, so where the allocator has no room for it this path still may
+    try {
+      if (packed_join(build, probe, compare_nulls, join_kind, a, out_probe, out_build)) return;
+    } catch (const Failure& f) {
+      if (f.code != GBX_ERR_ALLOC) throw;
+      for (gbx_column* c : {&out_probe, &out_build}) {
+        a.release(c->data, c->data_bytes);
+        std::memset(c, 0, sizeof(*c));
+      }
+    }
     const std::vector<gbx_column_view> bcols(build->columns, build->columns + build->num_columns);
     const std::vector<gbx_column_view> pcols(probe->columns, probe->columns + probe->num_columns);
     KeyTree tb = key_tree(bcols, GBX_NULL_INCLUDE);
@@ -414,8 +424,6 @@ int gbx_hash_join(const gbx_table_view* left, const gbx_table_view* right, int32
       GBX_CUDA(cudaMemsetAsync(matched, 0, std::max<int64_t>(nb, 1), s));
     }
     const bool pairs = join_kind != GBX_JOIN_LEFT_SEMI && join_kind != GBX_JOIN_LEFT_ANTI;
-    gbx_column& out_probe = swap ? *right_indices : *left_indices;
-    gbx_column& out_build = swap ? *left_indices : *right_indices;
     // the output size of a full join is known once the matches are marked
     int32_t* probe_buf = nullptr;
     int32_t* build_buf = nullptr;

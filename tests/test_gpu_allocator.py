@@ -97,3 +97,17 @@ def test_buffers_that_do_not_fit_in_one_piece_come_one_by_one():
     """20,000 rows: the sample's buffers together are 1.5 MB, the largest of them 1 MB."""
     k = np.arange(20_000, dtype=np.int64) % 100
     assert _sums(k, TightAllocator(1 << 20)) == {i: 200 for i in range(100)}
+
+
+@pytest.mark.parametrize("join", [J.inner_join, J.left_join, J.full_join], ids=["inner", "left", "full"])
+def test_join_where_the_packed_table_has_no_room(join):
+    """100,000 build rows: 4 MB of packed slots against 1 MB of row indices."""
+    rng = np.random.default_rng(9)
+    left, right = np.arange(150_000, dtype=np.int64)[::-1].copy(), rng.permutation(100_000).astype(np.int64)
+    pool = TightAllocator(2 << 20)
+    got = join(Table([T.device_column(HostCol(left))]), Table([T.device_column(HostCol(right))]), allocator=pool)
+    where = np.argsort(right)
+    want = [(i, int(where[k])) for i, k in enumerate(left) if k < 100_000]
+    if join is not J.inner_join:
+        want += [(i, J.JOIN_NONE) for i, k in enumerate(left) if k >= 100_000]
+    assert _pairs(got) == sorted(want)
