@@ -54,3 +54,19 @@ def test_packed_join_of_sliced_columns():
     where = {int(k): i for i, k in enumerate(b[7:390])}
     want = [(i, where[int(k)]) for i, k in enumerate(a[13:4111]) if int(k) in where]
     assert sorted(zip(li.tolist(), ri.tolist())) == want
+
+
+@pytest.mark.parametrize("nl,nr,card", [(1, 1, 1), (31, 4000, 3), (2048, 2500, 900), (2100, 3000, 30), (4097, 20_000, 50)])
+def test_repeated_keys_come_in_left_row_order(nl, nr, card):
+    """Each left row's pairs follow one another in row order; many outputs share a tile among several blocks."""
+    rng = np.random.default_rng(nl + nr)
+    left, right = rng.integers(0, card + 1, nl), rng.integers(0, card, nr)
+    right[0] = right[-1] = 0  # a repeated key
+    cols = [Table([T.device_column(HostCol(x.astype(np.int64)))]) for x in (left, right)]
+    li, ri = (c.to_numpy()[0] for c in J.left_join(*cols))
+    counts = np.bincount(right, minlength=card + 1)
+    assert np.array_equal(li, np.repeat(np.arange(nl), np.maximum(counts[left], 1)))
+    order = np.argsort(right, kind="stable")
+    first = np.cumsum(counts) - counts
+    want = np.concatenate([order[first[k]:first[k] + counts[k]] if counts[k] else [J.JOIN_NONE] for k in left])
+    assert np.array_equal(ri[np.lexsort((ri, li))], want)
