@@ -4,8 +4,8 @@
 // The general join (gbx_join.cu) stores build *row indices* in its table, so
 // a probe reads a slot, then the build key that row names: two dependent
 // random reads a probe, through the generic leaf comparison.  Here a 16-byte
-// slot holds the packed key itself beside the key's row count and first build
-// row, so a probe row is one 32-byte load in the usual case.  The probe is
+// slot holds the packed key itself beside the key's row count and a build
+// row of it, so a probe row is one 32-byte load in the usual case.  The probe is
 // bound by the L2's random-sector rate (the table of 1M build rows is 32 MB,
 // L2-resident); a thread keeps kJFlight loads in flight.
 //
@@ -43,17 +43,20 @@ constexpr int kJFlight           = 4;  // of which so many probe at a time
 constexpr int kJTile             = kJBlock * kJPer;
 constexpr uint32_t kNoSlot       = 0xffffffffu;
 // outputs of a block of k_pjoin_emit_runs: enough that the scan of its tile's
-// rows (2,048 lookups in the table) stays a small part of the work
-constexpr int64_t kEmitPart = 32768;
+// rows (2,048 lookups in the table) stays a small part of the work, or as few
+// as kEmitLeast while there are not two blocks an SM
+constexpr int64_t kEmitPart  = 32768;
+constexpr int64_t kEmitLeast = 2048;
 constexpr uintptr_t kSectorBytes = 32;  // a load_sector, aligned
-// build rows up to which a slot index (the reserved slot included) stays
-// below kNoSlot
+// build rows up to which a slot index and a representative (the reserved
+// slot's included) stay below kNoSlot
 constexpr int64_t kMaxBuildRows = int64_t(1) << 30;
 
-// One key of the build side: `first` is its first build row, and once
-// k_ranges has run on a table with repeated keys, the first position of its
-// rows in `rows`.  The all-ones word marks an empty slot; a key of all ones
-// has the reserved slot `cap`.  Slots are probed in pairs, each pair one
+// One key of the build side: `first` is a build row of it, the key's
+// representative (any one of its rows).  The all-ones word marks an
+// empty slot; a key of all ones has the reserved slot `cap` (and the
+// representative `n`, one past the build rows, since its slot is not claimed
+// by a compare-and-swap).  Slots are probed in pairs, each pair one
 // 32-byte sector: a key's home is a sector, and a probe examines a sector per
 // load (1.1 sectors a probe on average at the loads used, against 1.6 with
 // single slots; the probe is bound by the L2's random-sector rate).
@@ -116,72 +119,81 @@ __global__ void k_pjoin_clear(const PackedTable t)
     reinterpret_cast<uint4*>(t.slots)[s] = make_uint4(0xffffffffu, 0xffffffffu, 0u, 0u);
 }
 
-// Every build row's slot (kNoSlot: a row that matches nothing) and its rank
-// among its key's rows; the row of rank 0 is the slot's first.
+// Every build row's representative (kNoSlot: a row that matches nothing) and
+// its rank among its key's rows.  A new key's slot is claimed by one 128-bit
+// compare-and-swap that writes the key, the count 1 and the representative
+// together; a row of a known key adds 1 to the count and reads the
+// representative beside it, in one 64-bit add.  Each row so touches one
+// sector twice (20M unique keys, a 512 MB table: with the key claimed by
+// itself and the count and the row stored after it 2,057 us, the join by row
+// indices 933 us, this 1,397 us).
 template <int KM>
 __global__ void k_pjoin_build(const __grid_constant__ KeyPlan kp, int64_t n, const PackedTable t,
-                              uint32_t* __restrict__ slot_of, uint32_t* __restrict__ rank_of)
+                              uint32_t* __restrict__ rep_of, uint32_t* __restrict__ rank_of)
 {
+  bool repeated = false;  // stored once a thread: a store a repeated key, all to one address, would queue
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n;
        r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     uint64_t k;
     if (!row_key<KM>(kp, r, k)) {
-      slot_of[r] = kNoSlot;
+      rep_of[r] = kNoSlot;
       continue;
     }
-    uint64_t s = t.cap;
-    if (k != kEmptyWord) {
-      s = 2 * (fmix64(k) & (t.cap / 2 - 1));
-      for (uint64_t p = 0; p < t.cap; ++p) {  // cap > n: an empty slot is always met
-        unsigned long long* a = &t.slots[s].key;
-        unsigned long long cur = Global::ld_u64(reinterpret_cast<uint64_t>(a));
+    if (k == kEmptyWord) {
+      const uint32_t rank = atomicAdd(&t.slots[t.cap].cnt, 1u);
+      rep_of[r]           = static_cast<uint32_t>(n);
+      rank_of[r]          = rank;
+      if (rank == 0) t.slots[t.cap].first = static_cast<uint32_t>(r);
+      else repeated = true;
+      continue;
+    }
+    uint64_t s = 2 * (fmix64(k) & (t.cap / 2 - 1));
+    for (uint64_t p = 0; p < t.cap; ++p) {  // cap > n: an empty slot is always met
+      const uint64_t a = reinterpret_cast<uint64_t>(&t.slots[s].key);
+      uint64_t cur     = Global::ld_u64(a);
+      if (cur == kEmptyWord) {
+        uint64_t old;
+        Global::cas128(a, kEmptyWord, 0, k, (static_cast<uint64_t>(r) << 32) | 1u, cur, old);
         if (cur == kEmptyWord) {
-          cur = atomicCAS(a, static_cast<unsigned long long>(kEmptyWord), static_cast<unsigned long long>(k));
-          if (cur == kEmptyWord) break;
+          rep_of[r]  = static_cast<uint32_t>(r);
+          rank_of[r] = 0;
+          break;
         }
-        if (cur == k) break;
-        s = (s + 1) & (t.cap - 1);
       }
+      if (cur == k) {
+        // cnt (low half) and representative (high half)
+        const unsigned long long old = atomicAdd(reinterpret_cast<unsigned long long*>(a + 8), 1ULL);
+        rep_of[r]                    = static_cast<uint32_t>(old >> 32);
+        rank_of[r]                   = static_cast<uint32_t>(old);
+        repeated                     = true;
+        break;
+      }
+      s = (s + 1) & (t.cap - 1);
     }
-    const uint32_t rank = atomicAdd(&t.slots[s].cnt, 1u);
-    slot_of[r]          = static_cast<uint32_t>(s);
-    rank_of[r]          = rank;
-    if (rank == 0) t.slots[s].first = static_cast<uint32_t>(r);
-    else if (rank == 1) *t.dup = 1u;
+  }
+  if (repeated) *t.dup = 1u;
+}
+
+// With repeated keys: each key's row count at its representative (whose
+// exclusive scan places the keys' runs in `rows`), read off the slots: adding
+// the rows up again would queue on a key with many (1M rows of 100 keys 100 us).
+__global__ void k_pjoin_counts(const PackedTable t, int64_t n, uint32_t* __restrict__ cnt)
+{
+  for (uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s <= t.cap;
+       s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(t.slots) + s);
+    if (v.z != 0) cnt[s < t.cap ? v.w : static_cast<uint32_t>(n)] = v.z;
   }
 }
 
-// With repeated keys: each key's run of positions in `rows`, reserved warp by
-// warp from *cursor (the order of the runs does not matter).
-__global__ void k_pjoin_ranges(const PackedTable t, uint32_t* cursor)
+// The build rows of each key next to each other, from start_of[representative].
+__global__ void k_pjoin_place(int64_t n, const uint32_t* __restrict__ rep_of, const uint32_t* __restrict__ rank_of,
+                              const uint32_t* __restrict__ start_of, int32_t* __restrict__ rows)
 {
-  if (*t.dup == 0) return;
-  const int lane        = threadIdx.x & 31;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  const uint64_t n_up   = (t.cap + 1 + 31) & ~uint64_t(31);
-  for (uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s < n_up; s += stride) {
-    const uint32_t c = s <= t.cap ? t.slots[s].cnt : 0u;
-    uint32_t incl    = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    uint32_t base = 0;
-    if (lane == 31 && incl != 0) base = atomicAdd(cursor, incl);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    if (c != 0) t.slots[s].first = base + incl - c;
-  }
-}
-
-__global__ void k_pjoin_place(const PackedTable t, int64_t n, const uint32_t* __restrict__ slot_of,
-                              const uint32_t* __restrict__ rank_of, int32_t* __restrict__ rows)
-{
-  if (*t.dup == 0) return;
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n;
        r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint32_t s = slot_of[r];
-    if (s != kNoSlot) rows[t.slots[s].first + rank_of[r]] = static_cast<int32_t>(r);
+    const uint32_t k = rep_of[r];
+    if (k != kNoSlot) rows[start_of[k] + rank_of[r]] = static_cast<int32_t>(r);
   }
 }
 
@@ -339,9 +351,11 @@ __global__ void __launch_bounds__(kJBlock) k_pjoin_emit_one(const uint32_t* __re
 // after another (8 rows a thread; 1 row a thread in the join by row indices):
 // 10M probe rows of 4 pairs each 636 us (342), 100K of 1,000 2,646 us (1,916),
 // 2,000 of 10,000 24,756 us (3,217); here 182, 353 and 97 us.
-__global__ void __launch_bounds__(kJBlock) k_pjoin_emit_runs(const PackedTable t, const uint32_t* __restrict__ match,
+__global__ void __launch_bounds__(kJBlock) k_pjoin_emit_runs(const PackedTable t, int64_t nb,
+                                                             const uint32_t* __restrict__ match,
                                                              int64_t n, const int64_t* __restrict__ tile_at,
-                                                             int32_t kind, const int32_t* __restrict__ rows,
+                                                             int32_t kind, const uint32_t* __restrict__ start_of,
+                                                             const int32_t* __restrict__ rows,
                                                              int32_t* __restrict__ out_probe,
                                                              int32_t* __restrict__ out_build,
                                                              uint8_t* __restrict__ matched)
@@ -357,13 +371,17 @@ __global__ void __launch_bounds__(kJBlock) k_pjoin_emit_runs(const PackedTable t
   for (int q = 0; q < kJPer; ++q) {
     const int i      = threadIdx.x + q * kJBlock;
     const uint32_t m = r0 + i < n ? __ldg(match + r0 + i) : kNoSlot;
-    uint4 v          = make_uint4(0u, 0u, 0u, kNoSlot);
+    uint32_t cnt     = 0;
+    first[i]         = kNoSlot;
     if (m != kNoSlot) {
-      v = __ldg(reinterpret_cast<const uint4*>(t.slots) + m);
-      if (matched != nullptr && blockIdx.y == 0) matched[m] = 1;
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(t.slots) + m);
+      cnt           = v.z;
+      // (the reserved slot's representative is not in it)
+      const uint32_t rep = m == t.cap ? static_cast<uint32_t>(nb) : v.w;
+      first[i]           = __ldg(start_of + rep);
+      if (matched != nullptr && blockIdx.y == 0) matched[rep] = 1;
     }
-    start[i] = r0 + i < n ? rows_out(v.z, kind) : 0u;
-    first[i] = v.w;
+    start[i] = r0 + i < n ? rows_out(cnt, kind) : 0u;
   }
   __syncthreads();
   uint4* c         = reinterpret_cast<uint4*>(start) + threadIdx.x * 2;
@@ -411,16 +429,14 @@ __global__ void __launch_bounds__(kJBlock) k_pjoin_emit_runs(const PackedTable t
   }
 }
 
-// Full join: build rows whose key no probe row matched.  `matched` is indexed
-// by build row (unique keys) or by slot.
-__global__ void k_pjoin_unmatched(const uint32_t* __restrict__ slot_of, int64_t n, bool by_slot,
+// Full join: build rows whose key no probe row matched (`matched` is indexed
+// by build row when keys are unique, else by the key's representative).
+__global__ void k_pjoin_unmatched(const uint32_t* __restrict__ rep_of, int64_t n, bool repeated,
                                   const uint8_t* __restrict__ matched, uint32_t* __restrict__ flag)
 {
   for (int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; r < n;
-       r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint32_t s = slot_of[r];
-    flag[r]          = (s == kNoSlot || matched[by_slot ? s : static_cast<uint32_t>(r)] == 0) ? 1u : 0u;
-  }
+       r += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    flag[r] = (rep_of[r] == kNoSlot || matched[repeated ? rep_of[r] : static_cast<uint32_t>(r)] == 0) ? 1u : 0u;
 }
 
 __global__ void k_pjoin_append(const uint32_t* __restrict__ flag, const uint32_t* __restrict__ pos, int64_t n,
@@ -478,6 +494,28 @@ bool join_key_plans(const gbx_table_view* build, const gbx_table_view* probe, in
   return ok && kp.nwords == 1;
 }
 
+// Whether the packed table is the better one.  Its 16-byte slots are four times
+// the bytes that the join by row indices probes, so once they leave L2 its
+// build is the dearer one, and few probe rows do not earn that back.  Measured
+// on B200, whole left joins, packed / by row indices, us (unique keys; keys
+// drawn from as many as there are build rows):
+//   5M build rows (134 MB), probe rows 1,000    323 / 380    379 / 365
+//                                      nb / 8   338 / 431    407 / 425
+//   20M build rows (537 MB),           1,000  1,595 / 1,316  1,724 / 1,631
+//                                      nb / 8 1,688 / 1,572  1,869 / 1,848
+//                                      nb / 4 1,781 / 1,823  1,988 / 2,053
+//                                      nb     2,253 / 3,247  2,794 / 3,213
+//   50M build rows (1.07 GB, load 0.74),   nb / 2 7,597 / 7,132
+//                                          nb     9,087 / 10,210
+bool packed_pays(int64_t nb, int64_t np, uint64_t cap, size_t l2_bytes)
+{
+  const size_t bytes = cap * sizeof(Slot);
+  if (bytes <= l2_bytes) return true;
+  if (bytes <= 2 * l2_bytes) return 16 * np >= nb;
+  const bool loaded = 3 * static_cast<uint64_t>(nb) > 2 * cap;  // long probes
+  return bytes > 6 * l2_bytes && loaded ? 4 * np >= 3 * nb : 4 * np > nb;
+}
+
 }  // namespace
 
 bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32_t compare_nulls, int32_t kind,
@@ -487,11 +525,13 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   const int64_t np = probe->columns[0].size;
   KeyPlan kb{}, kp{};
   if (nb == 0 || np == 0 || nb > kMaxBuildRows || !join_key_plans(build, probe, compare_nulls, kb, kp)) return false;
-  cudaStream_t s    = a.st;
-  const int num_sms = current_device().num_sms;
+  cudaStream_t s       = a.st;
+  const DeviceInfo dev = current_device();
+  const int num_sms    = dev.num_sms;
   // load 0.375 to 0.75: at 1M build rows 32 MB of 16-byte slots, which stay
   // in L2 (a table twice that size does not fit beside the probe's streams)
   const uint64_t cap   = next_pow2(std::max<uint64_t>(static_cast<uint64_t>(nb) * 4 / 3 + 2, 64));
+  if (!packed_pays(nb, np, cap, dev.l2_bytes)) return false;
   const int64_t ntiles = (np + kJTile - 1) / kJTile;
 
   Scratch sc(&a);
@@ -502,33 +542,29 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   const size_t np4        = static_cast<size_t>(np) * 4;
   const size_t tile_bytes = static_cast<size_t>(ntiles + 1) * 8;
   size_t tb32 = 0, tb64 = 0;
-  GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, nb, nullptr, &tb32, s));
+  GBX_CUDA(scan_exclusive_u32(nullptr, nullptr, nb + 1, nullptr, &tb32, s));
   GBX_CUDA(scan_exclusive_i64(nullptr, nullptr, ntiles + 1, nullptr, &tb64, s));
   size_t tbytes = std::max(std::max(tb32, tb64), size_t(1));
-  sc.together({slot_bytes, 8, nb4, nb4, nb4, np4, tile_bytes, tbytes});
+  sc.together({slot_bytes, 8, nb4, nb4, np4, tile_bytes, tbytes});
   // 32-byte sectors, whatever the caller's allocator aligns to
   const auto raw = reinterpret_cast<uintptr_t>(sc.get(slot_bytes));
   t.slots        = reinterpret_cast<Slot*>((raw + kSectorBytes - 1) & ~(kSectorBytes - 1));
-  auto* flags   = static_cast<uint32_t*>(sc.get(8));  // repeated keys, cursor of the ranges
-  t.dup         = flags;
-  auto* slot_of = static_cast<uint32_t*>(sc.get(nb4));
+  t.dup         = static_cast<uint32_t*>(sc.get(8));
+  auto* rep_of  = static_cast<uint32_t*>(sc.get(nb4));
   auto* rank_of = static_cast<uint32_t*>(sc.get(nb4));
-  auto* rows    = static_cast<int32_t*>(sc.get(nb4));
   auto* match   = static_cast<uint32_t*>(sc.get(np4));
   auto* tiles   = static_cast<int64_t*>(sc.get(tile_bytes));
   void* temp    = sc.get(tbytes);
 
   // 1. the table
-  GBX_CUDA(cudaMemsetAsync(flags, 0, 8, s));
+  GBX_CUDA(cudaMemsetAsync(t.dup, 0, 8, s));
   k_pjoin_clear<<<grid_for(static_cast<int64_t>(cap) + 1, num_sms), kJBlock, 0, s>>>(t);
   const int gb = grid_for(nb, num_sms);
   switch (key_mode(kb)) {
-    case 1: k_pjoin_build<1><<<gb, kJBlock, 0, s>>>(kb, nb, t, slot_of, rank_of); break;
-    case 2: k_pjoin_build<2><<<gb, kJBlock, 0, s>>>(kb, nb, t, slot_of, rank_of); break;
-    default: k_pjoin_build<0><<<gb, kJBlock, 0, s>>>(kb, nb, t, slot_of, rank_of); break;
+    case 1: k_pjoin_build<1><<<gb, kJBlock, 0, s>>>(kb, nb, t, rep_of, rank_of); break;
+    case 2: k_pjoin_build<2><<<gb, kJBlock, 0, s>>>(kb, nb, t, rep_of, rank_of); break;
+    default: k_pjoin_build<0><<<gb, kJBlock, 0, s>>>(kb, nb, t, rep_of, rank_of); break;
   }
-  k_pjoin_ranges<<<grid_for(static_cast<int64_t>(cap) + 1, num_sms), kJBlock, 0, s>>>(t, flags + 1);
-  k_pjoin_place<<<gb, kJBlock, 0, s>>>(t, nb, slot_of, rank_of, rows);
   GBX_CUDA(cudaGetLastError());
 
   // 2. matches and output rows per tile
@@ -553,11 +589,25 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   const bool pairs = kind != GBX_JOIN_LEFT_SEMI && kind != GBX_JOIN_LEFT_ANTI;
   const bool one   = h_dup == 0 || !pairs;
   uint8_t* matched = nullptr;
+  uint32_t* start_of = nullptr;
+  int32_t* rows      = nullptr;
+  if (!one) {
+    // each key's rows next to each other (entry nb: the all-ones key)
+    sc.together({nb4 + 4, nb4 + 4, nb4});
+    auto* cnt = static_cast<uint32_t*>(sc.get(nb4 + 4));
+    start_of  = static_cast<uint32_t*>(sc.get(nb4 + 4));
+    rows      = static_cast<int32_t*>(sc.get(nb4));
+    GBX_CUDA(cudaMemsetAsync(cnt, 0, nb4 + 4, s));
+    k_pjoin_counts<<<grid_for(static_cast<int64_t>(cap) + 1, num_sms), kJBlock, 0, s>>>(t, nb, cnt);
+    GBX_CUDA(cudaGetLastError());
+    GBX_CUDA(scan_exclusive_u32(cnt, start_of, nb + 1, temp, &tbytes, s));
+    k_pjoin_place<<<gb, kJBlock, 0, s>>>(nb, rep_of, rank_of, start_of, rows);
+    GBX_CUDA(cudaGetLastError());
+  }
   int32_t *probe_buf = nullptr, *build_buf = nullptr;
   if (full) {
-    const size_t marks = h_dup ? static_cast<size_t>(cap) + 1 : static_cast<size_t>(nb);
-    matched            = static_cast<uint8_t*>(sc.get(marks));
-    GBX_CUDA(cudaMemsetAsync(matched, 0, marks, s));
+    matched = static_cast<uint8_t*>(sc.get(static_cast<size_t>(nb) + 1));
+    GBX_CUDA(cudaMemsetAsync(matched, 0, static_cast<size_t>(nb) + 1, s));
     probe_buf = static_cast<int32_t*>(sc.get(static_cast<size_t>(total) * 4));
     build_buf = static_cast<int32_t*>(sc.get(static_cast<size_t>(total) * 4));
   } else {
@@ -569,17 +619,20 @@ bool packed_join(const gbx_table_view* build, const gbx_table_view* probe, int32
   if (total > 0) {
     if (one) k_pjoin_emit_one<<<gp, kJBlock, 0, s>>>(match, np, tiles, kind, probe_buf, build_buf, matched);
     else {
-      // blocks a tile: one per kEmitPart outputs of the average tile
-      const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(total / ntiles / kEmitPart, 65535));
-      k_pjoin_emit_runs<<<dim3(gp, static_cast<unsigned>(parts)), kJBlock, 0, s>>>(t, match, np, tiles, kind, rows,
-                                                                                   probe_buf, build_buf, matched);
+      // blocks a tile: one per kEmitPart outputs of the average tile, more
+      // where that leaves SMs idle
+      const int64_t tile_out = total / ntiles;
+      const int64_t idle     = std::min<int64_t>((2 * num_sms + ntiles - 1) / ntiles, tile_out / kEmitLeast);
+      const int64_t parts    = std::max<int64_t>(1, std::min<int64_t>(std::max(tile_out / kEmitPart, idle), 65535));
+      k_pjoin_emit_runs<<<dim3(gp, static_cast<unsigned>(parts)), kJBlock, 0, s>>>(
+        t, nb, match, np, tiles, kind, start_of, rows, probe_buf, build_buf, matched);
     }
     GBX_CUDA(cudaGetLastError());
   }
   if (full) {
     auto* flag = static_cast<uint32_t*>(sc.get(nb4));
     auto* pos  = static_cast<uint32_t*>(sc.get(nb4));
-    k_pjoin_unmatched<<<gb, kJBlock, 0, s>>>(slot_of, nb, h_dup != 0, matched, flag);
+    k_pjoin_unmatched<<<gb, kJBlock, 0, s>>>(rep_of, nb, !one, matched, flag);
     GBX_CUDA(cudaGetLastError());
     GBX_CUDA(scan_exclusive_u32(flag, pos, nb, temp, &tbytes, s));
     uint32_t last[2] = {0, 0};

@@ -70,3 +70,31 @@ def test_repeated_keys_come_in_left_row_order(nl, nr, card):
     first = np.cumsum(counts) - counts
     want = np.concatenate([order[first[k]:first[k] + counts[k]] if counts[k] else [J.JOIN_NONE] for k in left])
     assert np.array_equal(ri[np.lexsort((ri, li))], want)
+
+
+@pytest.mark.parametrize("join", [J.inner_join, J.left_join, J.full_join], ids=["inner", "left", "full"])
+@pytest.mark.parametrize("repeated", [False, True], ids=["unique", "repeated"])
+@pytest.mark.parametrize("nl", [190_000, 230_000])
+def test_both_sides_of_the_line_for_tables_beyond_l2(nl, repeated, join):
+    """3.2M build rows (134 MB of slots): one probe row to 16 build rows is where the packed table begins to pay."""
+    rng = np.random.default_rng(nl)
+    nr = 3_200_000
+    right = rng.integers(0, nr, nr) if repeated else rng.permutation(nr)
+    left = rng.integers(0, nr + nr // 8, nl)
+    cols = [Table([T.device_column(HostCol(x.astype(np.int64)))]) for x in (left, right)]
+    li, ri = (c.to_numpy()[0].astype(np.int64) for c in join(*cols))
+    counts = np.bincount(right, minlength=nr + nr // 8)
+    order = np.argsort(right, kind="stable")
+    first = np.cumsum(counts) - counts
+    c = counts[left]
+    at = np.repeat(np.arange(nl), c)
+    want_l = at
+    want_r = order[first[left][at] + (np.arange(len(at)) - np.repeat(np.cumsum(c) - c, c))]
+    if join is not J.inner_join:
+        none = np.flatnonzero(c == 0)
+        want_l, want_r = np.concatenate([want_l, none]), np.concatenate([want_r, np.full(len(none), J.JOIN_NONE)])
+    if join is J.full_join:
+        rest = np.flatnonzero(~np.isin(right, left))
+        want_l, want_r = np.concatenate([want_l, np.full(len(rest), J.JOIN_NONE)]), np.concatenate([want_r, rest])
+    got, want = np.lexsort((ri, li)), np.lexsort((want_r, want_l))
+    assert np.array_equal(li[got], want_l[want]) and np.array_equal(ri[got], want_r[want])
