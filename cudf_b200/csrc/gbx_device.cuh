@@ -418,13 +418,18 @@ struct Global {
 // Linear probing over `mask + 1` slots starting at the hash's home slot.
 // Keys are stored as NW consecutive words per slot.  Returns the slot holding
 // `k` (inserting it into an empty slot if absent) or -1 when `max_probes`
-// slots were examined without success.  Every loop is bounded.
+// slots were examined without success, or (with `status`) a multiple of
+// kProbeStep while another key's failure has set S_TABLE_FULL there.  Every
+// loop is bounded.
+constexpr uint32_t kProbeStep = 64;  // far beyond a probe of a table that is not full
+
 template <class Space, int NW>
 __device__ __forceinline__ int64_t find_or_insert(typename Space::addr_t keys,
                                                   uint64_t mask,
                                                   const uint64_t (&k)[NW],
                                                   uint64_t h,
-                                                  uint32_t max_probes)
+                                                  uint32_t max_probes,
+                                                  const int32_t* status = nullptr)
 {
   uint64_t s = h & mask;
   for (uint32_t p = 0; p < max_probes; ++p) {
@@ -456,6 +461,9 @@ __device__ __forceinline__ int64_t find_or_insert(typename Space::addr_t keys,
           return static_cast<int64_t>(s);
       }
     }
+    if (status != nullptr && (p + 1) % kProbeStep == 0 &&
+        (Global::ld_u32(reinterpret_cast<uint64_t>(status)) & S_TABLE_FULL))
+      break;
     s = (s + 1) & mask;
   }
   return -1;

@@ -353,6 +353,12 @@ __device__ __forceinline__ void merge_slot(const Plan& plan,
 __device__ __forceinline__ Level<Global> global_level(const TableRef& t) { return Level<Global>{&t}; }
 
 // Global find-or-insert for one key, including the reserved all-ones slot.
+// -1 after max_probes slots, which sets S_TABLE_FULL; what the table holds is
+// then discarded and the pass redone with a larger one, so a key far from its
+// home gives up as soon as another has.  Without that every further row
+// examines max_probes slots, and where a warp waits for its lanes, so do the
+// rows beside it (20M rows of 845,000 groups in a table of 262,144: that pass
+// 38 ms one lane at a time, 88 ms by warps, 6 ms here).
 template <int NW>
 __device__ __forceinline__ int64_t global_slot(const TableRef& t,
                                                const uint64_t (&k)[NW],
@@ -362,8 +368,8 @@ __device__ __forceinline__ int64_t global_slot(const TableRef& t,
     if (Global::ld_u32(reinterpret_cast<uint64_t>(t.special_used)) == 0) atomicExch(t.special_used, 1u);
     return static_cast<int64_t>(t.cap);
   }
-  int64_t s = find_or_insert<Global, NW>(reinterpret_cast<uint64_t>(t.keys), t.cap - 1, k, hash_key<NW>(k),
-                                         max_probes);
+  const int64_t s = find_or_insert<Global, NW>(reinterpret_cast<uint64_t>(t.keys), t.cap - 1, k, hash_key<NW>(k),
+                                               max_probes, t.status);
   if (s < 0) atomicOr(t.status, S_TABLE_FULL);
   return s;
 }
