@@ -675,6 +675,43 @@ double estimate_groups(double sampled, double distinct, double heavy, double hea
 
 namespace {
 
+// Whether grouping tiles (gbx_tiled.cu) beats shared atomics a row
+// (k_agg_privatized) for a table of S slots with about `est` groups.  A tile
+// stages every value byte and folds a group's few rows as one chunk; a row
+// pays an atomic per accumulator (the floating ones are compare-and-swap
+// loops).  Up to 1,024 slots a tile holds enough rows of a group.  Measured on
+// B200, int64 keys, tiled / by rows at 80M rows (20M much the same; at 3M rows
+// tiled is at least as fast but for the plain COUNT):
+//                       520 groups  1,020   1,050  1,320  1,500  1,850  2,040
+//   COUNT                     1.05   0.98    1.26   1.40   1.49   1.52   1.65
+//   COUNT, nullable           1.06   0.98    0.89   1.03   1.10   1.17   1.28
+//   SUM int8                  1.01   0.96    0.72   0.85   0.90   0.97   1.10
+//   SUM int64, nullable       1.29   1.01    0.90   1.05   1.11   1.15   1.31
+//   SUM double, nullable      1.33   1.02    0.91   1.07   1.12   1.19   1.33
+//   MIN + MAX int32           0.93   0.89    0.64   0.75   0.80   0.86   1.00
+//   MIN + MAX double          1.22   1.17
+//   SUM of two int32          1.10   1.08
+//   SUM of two, one double    0.89   0.84
+//   SUM + MIN + MAX int64     0.56   0.61
+bool tiled_pays(const gbx::Plan& plan, uint32_t S, double est, int64_t n)
+{
+  if (S <= 1024 || plan.key.nwords > 1) return true;
+  int accs = plan.acc.nacc, staged = 0;  // accumulators but for the counts of valid rows, value bytes a row
+  bool loops = false, nullable = false;
+  for (int a = 0; a < plan.acc.nacc; ++a)
+    loops = loops || plan.acc.kind[a] == A_F64_ADD || plan.acc.kind[a] == A_F64_SHIFT ||
+            plan.acc.kind[a] == A_I64_MUL || plan.acc.kind[a] == A_F64_MUL;
+  for (int c = 0; c < plan.nchan; ++c) {
+    staged += pt_width(plan.chan[c].ptype);
+    if (plan.chan[c].a_cnt < 0) continue;
+    nullable = true;
+    --accs;
+  }
+  if (S <= 2048) return n < (int64_t(1) << 22) || staged < 8 || accs > (loops ? 1 : 2);
+  if (accs == 0 && !nullable) return false;
+  return n < (int64_t(1) << 24) || accs > 1 || est <= (nullable ? 1300.0 : 1900.0);
+}
+
 struct Call {
   gbx_groupby* gb;
   const gbx_request* reqs;
@@ -1435,7 +1472,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
           // a short probe: a hot key was inserted early and sits near its home
           // slot; a rare key that misses goes to the global table
           GBX_CUDA(launch_agg_tiled(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 8), max_probes, s));
-        } else if (tiled_fits(sl, plan) && !arg_kinds) {
+        } else if (tiled_fits(sl, plan) && !arg_kinds && tiled_pays(plan, S, est, call.n)) {
           // few groups: tiles grouped in shared memory before the table is touched
           GBX_CUDA(launch_agg_tiled(plan, t, sl, call.n, call.dev.num_sms, std::min<uint32_t>(S, 32), max_probes, s));
         } else {

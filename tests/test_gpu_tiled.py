@@ -55,3 +55,15 @@ def test_two_word_keys_and_dictionary_values(policy):
                 dict_keys=HostCol(np.array([-3, 8, 0, 77, 1 << 40], dtype=np.int64)))
     T.assert_parity(keys, [(d, SIX), (HostCol(rng.integers(0, 200, n).astype(np.uint8)), SIX)], policy,
                     Strategy.PRIVATIZED)
+
+
+@pytest.mark.parametrize("rows,groups", [(100_000, 1500), (4_200_000, 700), (17_000_000, 1250), (17_000_000, 1990)])
+def test_both_sides_of_the_line_to_atomics_a_row(rows, groups):
+    """Tables above 1,024 slots: few accumulators go by rows (gbx_abi.cpp, tiled_pays)."""
+    rng = np.random.default_rng(rows + groups)
+    k = HostCol(rng.integers(0, groups, rows).astype(np.int64))
+    v = HostCol(rng.integers(-100, 100, rows).astype(np.int64))
+    w = HostCol(rng.integers(0, 50, rows).astype(np.float64), rng.random(rows) >= 0.1)
+    for reqs in ([(v, [(Kind.COUNT_ALL, 0)])], [(v, [(Kind.SUM, 0)])], [(w, [(Kind.SUM, 0)])],
+                 [(w, [(Kind.MIN, 0), (Kind.MAX, 0)])], [(v, [(Kind.SUM, 0), (Kind.MIN, 0), (Kind.MAX, 0)])]):
+        T.assert_parity([k], reqs)
