@@ -976,9 +976,10 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     int launches = 0;
     timer.mark(0);
     // control block: [0..1] sample counters, [2..25] valid counts, [26] status,
-    // [27] num_selected, [28..31] partitioned-path counters, [32..33] heavy keys
-    // of the sample and their rows, then the outputs' null counters
-    constexpr int kNullsAt  = 34;
+    // [27] num_selected, [28..31] partitioned-path counters, [32..34] heavy keys
+    // of the sample, their rows, the most rows of one key, then the outputs'
+    // null counters
+    constexpr int kNullsAt  = 35;
     constexpr int kCtlWords = kNullsAt + kMaxKeyCols + kMaxOut;
     static_assert(kCtlWords * 8 <= kReadbackBytes, "the control block fits the read-back buffer");
     const int64_t nsample  = std::min<int64_t>(call.n, 1 << 16);
@@ -1052,15 +1053,25 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     constexpr int64_t kBucketedMinRows = int64_t(1) << 22;
     int bucket_bits       = 0;
     uint32_t bucket_slots = 0;
-    for (int bb : {8, 16}) {
-      const double groups = est / (2.0 * call.dev.num_sms) + est / static_cast<double>(1u << bb);
+    auto fit_buckets      = [&](int bb, bool two_per_sm) {
+      const double runs   = (two_per_sm ? 2.0 : 1.0) * call.dev.num_sms;
+      const double groups = est / runs + est / static_cast<double>(1u << bb);
       const auto Sb = static_cast<uint32_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * groups, 64.0))));
-      if (Sb <= 1024 && tiled_fits(make_smem_layout(plan, Sb), plan, /*two_per_sm=*/true)) {
-        bucket_bits  = bb;
-        bucket_slots = Sb;
-        break;
-      }
-    }
+      if (Sb > (two_per_sm ? 1024u : 512u) || !tiled_fits(make_smem_layout(plan, Sb), plan, two_per_sm)) return false;
+      bucket_bits  = bb;
+      bucket_slots = Sb;
+      return true;
+    };
+    // one run an SM in one pass rather than two in two passes (30M rows, 3e4
+    // groups, three nullable doubles of six kinds: 3.1 against 3.7 ms)
+    if (!fit_buckets(8, true) && fit_buckets(16, true)) fit_buckets(8, false);
+    // A plan too wide for two CTAs an SM goes to the global table (30M rows,
+    // five nullable doubles, 1e4 even groups: 2.2 ms, one run an SM 3.1) unless
+    // one key holds 2% of the rows or more, on whose slot the global table's
+    // atomics would queue (Zipf 1.02, a hottest key of 10%: 6.4 ms, one run an
+    // SM 3.7).
+    const double hottest = h_ctl[0] > 0 ? static_cast<double>(h_ctl[34]) / static_cast<double>(h_ctl[0]) : 0.0;
+    if (bucket_bits == 0 && hottest >= 0.02) fit_buckets(8, false);
     int strategy = gb->strategy;
     if (strategy == GBX_STRATEGY_BUCKETED && bucket_bits == 0) {
       // forced with more groups than a tiled table holds: the largest table
@@ -1083,6 +1094,19 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       const auto need = static_cast<uint32_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * s_heavy, 64.0))));
       if (need <= 4096 && tiled_fits(make_smem_layout(plan, need), plan)) stream_slots = need;
     }
+    // A wide plan's table leaves room for few rows beside it, so that most of a
+    // chunk's work is merging it: beyond this many shared atomics a row the
+    // bucket-ordered rows are the faster way, where they are one.  Measured on
+    // B200, 30M rows, this / bucketed: five nullable doubles (SUM, COUNT, MEAN),
+    // 1,000 groups (10 a row) 5.6 / 3.0 ms; three (all six kinds), 300 groups
+    // (6.2) 4.0 / 2.6; eight int8, 1,000 groups (2.6) 2.9 / 2.1; five doubles,
+    // 1,000 groups (2.4) 2.8 / 2.2; four nullable doubles, 600 groups (2.35)
+    // 2.1 / 2.6; two (all six), 300 groups (1.4) 1.2 / 1.7.
+    bool skew_bucketed = false;
+    if (strategy == GBX_STRATEGY_AUTO && stream_slots > 0 && bucket_bits > 0 && call.n >= kBucketedMinRows && global_in_l2) {
+      const double rows_a_group = tiled_rows(make_smem_layout(plan, stream_slots), plan) / std::max(s_heavy, 1.0);
+      skew_bucketed             = nacc / std::max(1.0, std::min(rows_a_group, 16.0)) > 2.4;
+    }
     bool skew_stream = false;
     if (strategy == GBX_STRATEGY_AUTO) {
       // measured on B200 (100M rows, 12 accumulators): at 100 groups the shared
@@ -1091,8 +1115,8 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       // path 21.4 ms; at 1e6 groups (table beyond L2) 32.6 ms against 17.2 ms
       if (est * 2.0 <= static_cast<double>(s_max)) strategy = GBX_STRATEGY_PRIVATIZED;
       else if (stream_slots > 0) {
-        strategy    = GBX_STRATEGY_PRIVATIZED;
-        skew_stream = true;
+        strategy    = skew_bucketed ? GBX_STRATEGY_BUCKETED : GBX_STRATEGY_PRIVATIZED;
+        skew_stream = !skew_bucketed;
         // the rare keys land in the global table: room for more of them than
         // the sample saw
         cap = std::min<uint64_t>(cap * 4, 1ULL << 31);
@@ -1526,9 +1550,13 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       const uint64_t bound = next_pow2(2 * static_cast<uint64_t>(call.n) + 2);
       cap = std::min<uint64_t>(attempt == 0 ? std::min<uint64_t>(cap * 16, bound) : std::max<uint64_t>(cap * 4, bound),
                                1ULL << 31);
-      if (strategy == GBX_STRATEGY_WARP || strategy == GBX_STRATEGY_BUCKETED ||
-          (strategy == GBX_STRATEGY_PRIVATIZED && !skew_stream))
+      if (strategy == GBX_STRATEGY_BUCKETED && skew_bucketed) {
+        strategy    = GBX_STRATEGY_PRIVATIZED;
+        skew_stream = true;
+      } else if (strategy == GBX_STRATEGY_WARP || strategy == GBX_STRATEGY_BUCKETED ||
+                 (strategy == GBX_STRATEGY_PRIVATIZED && !skew_stream)) {
         strategy = GBX_STRATEGY_GLOBAL;
+      }
       est = static_cast<double>(cap / 2);
     }
     gb->stats.strategy        = strategy;

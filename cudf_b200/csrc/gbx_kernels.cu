@@ -172,17 +172,28 @@ __global__ void k_sample_distinct(const __grid_constant__ KeyPlan kp,
 }
 
 // Keys sampled at least kHeavySample times: heavy[0] += their number,
-// heavy[1] += their sampled rows.
+// heavy[1] += their sampled rows; heavy[2] = the most rows of one key.
 __global__ void k_sample_heavy(const uint32_t* set_rows, uint64_t set_cap, unsigned long long* heavy)
 {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  uint32_t keys = 0, rows = 0, most = 0;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < set_cap; i += stride) {
     const uint32_t c = set_rows[i];
+    most             = max(most, c);
     if (c >= kHeavySample) {
-      atomicAdd(&heavy[0], 1ULL);
-      atomicAdd(&heavy[1], static_cast<unsigned long long>(c));
+      ++keys;
+      rows += c;
     }
   }
+  keys = __reduce_add_sync(0xffffffffu, keys);
+  rows = __reduce_add_sync(0xffffffffu, rows);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) != 0 || most == 0) return;
+  if (keys != 0) {
+    atomicAdd(&heavy[0], static_cast<unsigned long long>(keys));
+    atomicAdd(&heavy[1], static_cast<unsigned long long>(rows));
+  }
+  atomicMax(&heavy[2], static_cast<unsigned long long>(most));
 }
 
 // Empties the sample's set, its row counts and the counters of both.
@@ -195,10 +206,8 @@ __global__ void k_clear_sample(uint64_t* set, uint32_t* rows, uint64_t n, unsign
     set[i]  = kEmptyWord;
     rows[i] = 0;
   }
-  if (i0 < 2) {
-    counters[i0] = 0;
-    heavy[i0]    = 0;
-  }
+  if (i0 < 2) counters[i0] = 0;
+  if (i0 < 3) heavy[i0] = 0;
 }
 
 // ------------------------------------------------------------- finalize

@@ -43,7 +43,8 @@ struct OutPlan {
 cudaError_t launch_init_table(const TableRef& t, const AccLayout& al, int nwords, int num_sms, cudaStream_t st);
 // Sampled distinct count of nsample strided rows: counters[0] = sampled rows,
 // counters[1] = their distinct keys; heavy[0] = keys sampled at least
-// kHeavySample times, heavy[1] = their sampled rows.  `set` holds set_cap
+// kHeavySample times, heavy[1] = their sampled rows, heavy[2] = the most
+// sampled rows of one key.  `set` holds set_cap
 // words and `set_rows` set_cap counts (set_cap a power of two).
 constexpr uint32_t kHeavySample = 4;
 cudaError_t launch_sample(const KeyPlan& kp, int64_t n, int64_t nsample, uint64_t* set, uint32_t* set_rows,
@@ -58,6 +59,8 @@ cudaError_t launch_agg_privatized(const Plan& p, const TableRef& t, const SmemLa
 // and a tile's staged values within an SM's shared memory, or within half of
 // it with two_per_sm).
 bool tiled_fits(const SmemLayout& sl, const Plan& p, bool two_per_sm = false);
+// Rows of a tile (0: no tile fits).
+int tiled_rows(const SmemLayout& sl, const Plan& p);
 cudaError_t launch_agg_tiled(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int num_sms,
                              uint32_t smem_probes, uint32_t max_probes, cudaStream_t st);
 // ---- radix-partitioned path

@@ -703,6 +703,11 @@ bool tiled_fits(const SmemLayout& sl, const Plan& p, bool two_per_sm)
   return tl.tile_rows > 0 && (!two_per_sm || tl.block == 512);
 }
 
+int tiled_rows(const SmemLayout& sl, const Plan& p)
+{
+  return sl.slots > static_cast<uint32_t>(kMaxSlots) ? 0 : pick_tiled_layout(sl, p).tile_rows;
+}
+
 cudaError_t launch_agg_tiled(const Plan& p, const TableRef& t, const SmemLayout& sl, int64_t n, int num_sms,
                              uint32_t smem_probes, uint32_t max_probes, cudaStream_t st)
 {

@@ -67,3 +67,17 @@ def test_both_sides_of_the_line_to_atomics_a_row(rows, groups):
     for reqs in ([(v, [(Kind.COUNT_ALL, 0)])], [(v, [(Kind.SUM, 0)])], [(w, [(Kind.SUM, 0)])],
                  [(w, [(Kind.MIN, 0), (Kind.MAX, 0)])], [(v, [(Kind.SUM, 0), (Kind.MIN, 0), (Kind.MAX, 0)])]):
         T.assert_parity([k], reqs)
+
+
+@pytest.mark.parametrize("rows,groups,hot", [(4_200_000, 300, 0.0), (4_200_000, 300, 0.3), (4_200_000, 3_000, 0.0),
+                                             (4_200_000, 12_000, 0.015), (4_200_000, 12_000, 0.1), (4_200_000, 40_000, 0.1)])
+def test_wide_plans_and_a_hot_key(rows, groups, hot):
+    """Plans too wide for two tables an SM: bucketed, one run an SM, the global table, or the skewed form."""
+    rng = np.random.default_rng(groups)
+    k = rng.integers(0, groups, rows).astype(np.int64)
+    k[rng.random(rows) < hot] = groups // 2
+    vals = [HostCol(rng.integers(-99, 99, rows).astype(np.float64), rng.random(rows) >= 0.1) for _ in range(5)]
+    for aggs, cols in (([(Kind.SUM, 0), (Kind.COUNT_VALID, 0), (Kind.MEAN, 0)], vals),
+                       ([(Kind.SUM, 0), (Kind.MIN, 0), (Kind.MAX, 0), (Kind.VARIANCE, 1)], vals[:3])):
+        got, _ = T.assert_parity([HostCol(k)], [(v, aggs) for v in cols])
+        assert got["stats"]["retries"] == 0
