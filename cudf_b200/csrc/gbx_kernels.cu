@@ -409,7 +409,8 @@ cudaError_t launch_sample(const KeyPlan& kp, int64_t n, int64_t nsample, uint64_
   int grid = grid_for(nsample, 256, num_sms * 8);
   if (kp.nwords == 1) k_sample_distinct<1><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
   else k_sample_distinct<2><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
-  k_sample_heavy<<<fill_grid, 256, 0, st>>>(set_rows, set_cap, heavy);
+  // few warps, whose sums queue on three words
+  k_sample_heavy<<<grid_for(static_cast<int64_t>(set_cap), 256, num_sms), 256, 0, st>>>(set_rows, set_cap, heavy);
   return cudaGetLastError();
 }
 
