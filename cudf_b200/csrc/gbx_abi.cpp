@@ -984,8 +984,13 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     static_assert(kCtlWords * 8 <= kReadbackBytes, "the control block fits the read-back buffer");
     const int64_t nsample  = std::min<int64_t>(call.n, 1 << 16);
     const uint64_t set_cap = next_pow2(4 * static_cast<uint64_t>(nsample));  // 2^18 from 65,536 rows on
-    scratch.together({kCtlWords * 8, set_cap * 8, set_cap * 4});
+    // the sample's set is free again once its counts are read: the table and
+    // what follows take its room, and a small call some beside it
+    const size_t room =
+      nsample < (1 << 16) ? std::min<size_t>((size_t(3) << 20) - set_cap * 12, (128 << 10) + 64 * call.n) : 0;
+    scratch.together({kCtlWords * 8, set_cap * 8, set_cap * 4, room});
     auto* ctl = static_cast<unsigned long long*>(scratch.get(kCtlWords * 8));
+    const size_t after_ctl = scratch.mark();
     GBX_CUDA(cudaMemsetAsync(ctl, 0, kCtlWords * 8, s));
     int32_t* d_status        = reinterpret_cast<int32_t*>(ctl + 26);
     int64_t* d_num_selected  = reinterpret_cast<int64_t*>(ctl + 27);
@@ -1011,6 +1016,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       GBX_CUDA(cudaStreamSynchronize(s));
     };
     read_ctl();
+    scratch.rewind(after_ctl);
     for (size_t i = 0; i < span_owner.size(); ++i) {
       int64_t nulls = static_cast<int64_t>(ms.span[i].size) - static_cast<int64_t>(h_ctl[2 + i]);
       if (span_owner[i].first == 0) key_nulls[span_owner[i].second] = nulls;

@@ -128,6 +128,7 @@ struct Scratch {
   {
     size_t sum = 0;
     for (size_t b : sizes) sum += rounded(b) <= kSmall ? rounded(b) : 0;
+    if (used + sum <= block_bytes) return;
     block = nullptr;
     used = block_bytes = 0;
     if (sum == 0) return;
@@ -138,6 +139,10 @@ struct Scratch {
       // no room for them in one piece: one by one
     }
   }
+  // The buffers carved since mark() are free again (for work that follows
+  // theirs on the stream); no together() in between.
+  size_t mark() const { return used; }
+  void rewind(size_t m) { used = m; }
   size_t total() const
   {
     size_t s = 0;
