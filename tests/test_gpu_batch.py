@@ -244,3 +244,31 @@ def test_dictionary_values_in_a_batch():
         insts.append(([HostCol(k)], [(HostCol(idx, dict_keys=dk), [(Kind.SUM, 0), (Kind.MIN, 0), (Kind.MEAN, 0)])]))
     _, _, res = run_batch(insts)
     check_batch(insts, res)
+
+
+def _many_columns(n_inst, columns, seed, two_words=False):
+    rng = np.random.default_rng(seed)
+    insts = []
+    for i in range(n_inst):
+        n = int(10 ** rng.uniform(2, 4.5))
+        card = int(10 ** rng.uniform(0.7, 3.7))
+        keys = [HostCol(rng.integers(0, card, n, dtype=np.int64))]
+        if two_words:
+            keys.append(HostCol(rng.integers(0, 2, n, dtype=np.int64)))
+        reqs = []
+        for c in range(columns):
+            dt = (np.int64, np.float64, np.int32, np.float32, np.int16)[c % 5]
+            v = rng.integers(-100, 100, n).astype(dt)
+            reqs.append((HostCol(v, (rng.random(n) > 0.1) if c % 2 else None),
+                         [(Kind.SUM, 0), (Kind.MAX, 0), (Kind.COUNT_VALID, 0)]))
+        insts.append((keys, reqs))
+    return insts
+
+
+@pytest.mark.parametrize("two_words", [False, True], ids=["one_word", "two_words"])
+@pytest.mark.parametrize("block", [256, 512])
+@pytest.mark.parametrize("mode", MODES, ids=lambda m: m.name)
+def test_more_than_two_columns(mode, block, two_words):
+    insts = _many_columns(16, 3 if two_words else 6, seed=block + int(mode), two_words=two_words)
+    _, _, res = run_batch(insts, force_mode=mode, block_threads=block)
+    check_batch(insts, res)
