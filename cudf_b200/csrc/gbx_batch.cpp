@@ -34,8 +34,10 @@ namespace {
 // two CTAs an SM and 1,024 with one: a table beyond half an SM's shared memory
 // leaves room for one CTA, which then needs all the threads (measured on the
 // class of 1,024-2,047 groups: 512 threads 54 G rows/s, 1,024 90 G).  256
-// threads, at most 100 KB each, measured below both in every class; a caller
-// may still ask for them.
+// threads, at most 100 KB each, measured below the better of the two in every
+// class (and above 1,024 in one, of 16-31 groups: 148.1 against 147.0 G
+// rows/s); a caller may still ask for them.  Without measurements a batch runs
+// on 512.
 constexpr size_t kSmemBudget256  = 100 * 1024;
 constexpr size_t kSmemBudgetBig  = kBatchMaxDynamicSmem;
 constexpr int kSamplePerInstance = 2048;
@@ -47,7 +49,7 @@ size_t smem_budget(int block) { return block >= 512 ? kSmemBudgetBig : kSmemBudg
 // One tuned choice for a class of instances under one block shape.
 struct Choice {
   int32_t mode      = BM_GLOBAL;
-  int32_t smul      = 0;   // shared table slots = base_slots(class) * 2^smul, smul -1 to 2
+  int32_t smul      = 0;   // shared table slots = choice_slots(class, smul), smul -1 to 2
   int32_t tile_log2 = 16;  // rows per work item
   double rate       = 0;   // measured rows/s of the class (0: not measured)
 };
@@ -60,17 +62,18 @@ int class_of(double est)
   return c;
 }
 
-// Slots of a shared-memory table for a class at load <= 0.8 of its largest
-// member (groups < 2^(cls+1)).
+// Slots of a shared-memory table for a class: the power of two above 1.25
+// times its largest member's groups (< 2^(cls+1)), that is twice them: load
+// <= 0.5.
 uint32_t base_slots(int cls)
 {
   uint64_t s = next_pow2(static_cast<uint64_t>(std::ceil(std::ldexp(1.0, cls + 1) * 1.25)));
   return static_cast<uint32_t>(std::max<uint64_t>(s, 32));
 }
 
-// Slots under a choice.  smul -1 loads the table up to 1.25 times its slots
-// at the class's upper end (the rows of the last groups then go to the global
-// table): it still wins for classes whose full table does not fit.
+// Slots under a choice.  smul -1 loads the table up to 1.0 at the class's
+// upper end (rows whose group finds no slot within the probe limit go to the
+// global table): it still wins for classes whose full table does not fit.
 uint32_t choice_slots(int cls, int smul)
 {
   const uint32_t s = base_slots(cls);
@@ -737,6 +740,7 @@ void plan_batch(gbx_batch& b, const gbx_batch_options& o)
         std::vector<Choice> cand;
         for (int tl : {15, 17}) {
           for (int smul = -1; smul <= 1; ++smul) {
+            if (smul == 0 && choice_slots(cls, -1) == choice_slots(cls, 0)) continue;  // the smallest table
             Choice c;
             c.mode = BM_SHARED, c.smul = smul, c.tile_log2 = tl;
             cand.push_back(c);

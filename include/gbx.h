@@ -445,7 +445,7 @@ typedef struct gbx_batch_options {
   int32_t tune;                /* gbx_batch_tune */
   const char* tune_file;       /* the persisted tuning table (NULL: none) */
   int32_t force_mode;          /* gbx_batch_mode for every instance (AUTO: per instance) */
-  int32_t block_threads;       /* 0: tuner's choice; else 256 or 512 */
+  int32_t block_threads;       /* 0: tuner's choice (512 or 1,024; 512 without measurements); else 256 or 512 */
   int32_t one_shot;            /* 1: launch the kernels directly at execute instead of capturing a
                                   graph (cheaper for a batch that runs once) */
   int64_t tile_rows;           /* 0: tuner's choice; else rows per work item */

@@ -272,3 +272,50 @@ def test_more_than_two_columns(mode, block, two_words):
     insts = _many_columns(16, 3 if two_words else 6, seed=block + int(mode), two_words=two_words)
     _, _, res = run_batch(insts, force_mode=mode, block_threads=block)
     check_batch(insts, res)
+
+
+def _near_full(n_inst, two_words, columns):
+    """Instances whose group counts sit near a class's upper end, so that a table of half the class's size is nearly
+    full and some rows find no slot within its probe limit."""
+    rng = np.random.default_rng(77)
+    insts = []
+    for i in range(n_inst):
+        card = (1 << (6 + i % 5)) * 15 // 16
+        n = 12 * card + int(rng.integers(0, 999))
+        k = rng.permutation(np.arange(n, dtype=np.int64) % card)
+        keys = [HostCol(k * 3 - 1)]
+        if two_words:
+            keys.append(HostCol(-k))
+        insts.append((keys, [(HostCol(rng.integers(-99, 99, n).astype((np.int64, np.float64, np.int32)[c % 3]),
+                                      (rng.random(n) > 0.1) if c == 1 else None), SUM_COUNT_MAX)
+                             for c in range(columns)]))
+    return insts
+
+
+@pytest.mark.parametrize("columns", [1, 4])
+@pytest.mark.parametrize("two_words", [False, True], ids=["one_word", "two_words"])
+@pytest.mark.parametrize("mode,smul", [(BatchMode.SHARED, -1), (BatchMode.SHARED, 0), (BatchMode.SHARED, 1),
+                                       (BatchMode.WARP, 0), (BatchMode.GLOBAL, 0)],
+                         ids=["half", "full", "twice", "warp", "global"])
+def test_blocks_of_1024_threads_from_a_tuning_table(tmp_path, mode, smul, two_words, columns):
+    """The 1,024-thread shape, which only a tuning table chooses, in every mode and table size."""
+    insts = _near_full(20, two_words, columns)
+    path = str(tmp_path / "tune.txt")
+    run_batch(insts[:5], tune=Tune.MISSING, tune_file=path)  # the lines' device, schema and classes
+    lines = [l.split() for l in open(path).read().splitlines() if l.strip()]
+    with open(path, "w") as f:
+        for l in lines:
+            rate = 10 ** 12 if l[2] == "1024" else 10 ** 6
+            f.write(" ".join(l[:4] + [str(int(mode)), str(smul), "15", str(rate)]) + "\n")
+    b, _, res = run_batch(insts, tune=Tune.CACHED, tune_file=path)
+    st = b.stats()
+    assert st["block_threads"] == 1024 and st["classes_measured"] == 0 and st["classes_cached"] == 2 * st["classes"]
+    plan = b.instance_plan()
+    # a table that does not fit shared memory falls back to the global one
+    assert np.all((plan["mode"] == int(mode)) | (plan["mode"] == int(BatchMode.GLOBAL)))
+    assert (plan["mode"] == int(mode)).any()
+    if smul == -1:
+        assert np.all(plan["mode"] == int(mode))
+        assert (plan["table_slots"] <= 1.25 * plan["estimated_groups"]).all()
+    check_batch(insts, res)
+    check_batch(insts, b.execute())
