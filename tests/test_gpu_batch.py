@@ -274,13 +274,13 @@ def test_more_than_two_columns(mode, block, two_words):
     check_batch(insts, res)
 
 
-def _near_full(n_inst, two_words, columns):
+def _near_full(n_inst, two_words, columns, octave):
     """Instances whose group counts sit near a class's upper end, so that a table of half the class's size is nearly
     full and some rows find no slot within its probe limit."""
     rng = np.random.default_rng(77)
     insts = []
     for i in range(n_inst):
-        card = (1 << (6 + i % 5)) * 15 // 16
+        card = (1 << (octave + i % 5)) * 15 // 16
         n = 12 * card + int(rng.integers(0, 999))
         k = rng.permutation(np.arange(n, dtype=np.int64) % card)
         keys = [HostCol(k * 3 - 1)]
@@ -299,7 +299,7 @@ def _near_full(n_inst, two_words, columns):
                          ids=["half", "full", "twice", "warp", "global"])
 def test_blocks_of_1024_threads_from_a_tuning_table(tmp_path, mode, smul, two_words, columns):
     """The 1,024-thread shape, which only a tuning table chooses, in every mode and table size."""
-    insts = _near_full(20, two_words, columns)
+    insts = _near_full(20, two_words, columns, 2 if mode == BatchMode.WARP else 6)  # 32 warps' tables are small ones
     path = str(tmp_path / "tune.txt")
     run_batch(insts[:5], tune=Tune.MISSING, tune_file=path)  # the lines' device, schema and classes
     lines = [l.split() for l in open(path).read().splitlines() if l.strip()]
