@@ -103,10 +103,13 @@ struct Alloc {
 // Scratch buffers released (stream-ordered) when the owner goes away.  A call
 // takes a dozen small ones, and a caller's allocator costs microseconds each
 // (a 10K-row call spends most of its time on the host), so sizes known
-// together() share one allocation of exactly their sum: fewer allocations,
-// and no more memory than one each.
+// together() share one allocation of their sum and kSlack, from which the
+// control words and the like that follow are carved too.  Where the allocator
+// refuses that, the buffers come one by one.
 struct Scratch {
   static constexpr size_t kSmall = size_t(2) << 20;  // a buffer beyond this is allocated by itself
+  static constexpr size_t kTiny  = 4096;             // a buffer up to this is always carved
+  static constexpr size_t kSlack = 32768;
   Alloc* a;
   std::vector<std::pair<void*, size_t>> bufs;
   unsigned char* block = nullptr;  // the allocation being carved
@@ -118,6 +121,7 @@ struct Scratch {
   void* get(size_t bytes)
   {
     const size_t need = rounded(bytes);
+    if (need <= kTiny && used + need > block_bytes) together({bytes});
     if (need > kSmall || used + need > block_bytes) return own(bytes);
     void* p = block + used;
     used += need;
@@ -133,10 +137,10 @@ struct Scratch {
     used = block_bytes = 0;
     if (sum == 0) return;
     try {
-      block       = static_cast<unsigned char*>(own(sum));
-      block_bytes = sum;
+      block       = static_cast<unsigned char*>(own(sum + kSlack));
+      block_bytes = sum + kSlack;
     } catch (const Failure&) {
-      // no room for them in one piece: one by one
+      // no room for them in one piece
     }
   }
   // The buffers carved since mark() are free again (for work that follows

@@ -7,8 +7,10 @@ import numpy as np
 import pytest
 
 from cudf_b200 import Column, GroupBy, GroupByRequest, Table
+from cudf_b200 import _lib
 from cudf_b200 import aggregation as agg
 from cudf_b200 import join as J
+from cudf_b200._abi import Status
 from cudf_b200.groupby import TorchAllocator
 from oracle.oracle import HostCol
 from tests import gbx_testing as T
@@ -111,3 +113,17 @@ def test_join_where_the_packed_table_has_no_room(join):
     if join is not J.inner_join:
         want += [(i, J.JOIN_NONE) for i, k in enumerate(left) if k >= 100_000]
     assert _pairs(got) == sorted(want)
+
+
+@pytest.mark.parametrize("room", [48 << 10, 100 << 10, 300 << 10, 1 << 20])
+def test_a_join_in_a_pool_of_a_few_buffers(room):
+    """A pool too small for the shared allocation still serves what fits buffer by buffer, or says that it cannot."""
+    left, right = np.arange(2000, dtype=np.int64), np.arange(1000, dtype=np.int64)
+    pool = TightAllocator(room, room)
+    tables = [Table([T.device_column(HostCol(x))]) for x in (left, right)]
+    try:
+        got = J.inner_join(*tables, allocator=pool)
+    except _lib.GbxError as e:
+        assert e.status == Status.ERR_ALLOC and room < 100 << 10
+    else:
+        assert _pairs(got) == [(i, i) for i in range(1000)]
