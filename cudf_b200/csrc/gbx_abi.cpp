@@ -1098,10 +1098,10 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     const double s_heavy = static_cast<double>(h_ctl[32]), s_heavy_rows = static_cast<double>(h_ctl[33]);
     const bool skewed    = h_ctl[0] > 0 && s_heavy_rows >= 0.75 * static_cast<double>(h_ctl[0]);
     // its table: twice the heavy keys (one CTA an SM when it does not fit two)
-    uint32_t stream_slots = 0;
+    uint32_t skew_slots = 0;
     if (skewed && !plan_has_arg(plan)) {
       const auto need = static_cast<uint32_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * s_heavy, 64.0))));
-      if (need <= 4096 && tiled_fits(make_smem_layout(plan, need), plan)) stream_slots = need;
+      if (need <= 4096 && tiled_fits(make_smem_layout(plan, need), plan)) skew_slots = need;
     }
     // A wide plan's table leaves room for few rows beside it, so that most of a
     // chunk's work is merging it: beyond this many shared atomics a row the
@@ -1112,20 +1112,21 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     // 1,000 groups (2.4) 2.8 / 2.2; four nullable doubles, 600 groups (2.35)
     // 2.1 / 2.6; two (all six), 300 groups (1.4) 1.2 / 1.7.
     bool skew_bucketed = false;
-    if (strategy == GBX_STRATEGY_AUTO && stream_slots > 0 && bucket_bits > 0 && call.n >= kBucketedMinRows && global_in_l2) {
-      const double rows_a_group = tiled_rows(make_smem_layout(plan, stream_slots), plan) / std::max(s_heavy, 1.0);
+    if (strategy == GBX_STRATEGY_AUTO && skew_slots > 0 && bucket_bits > 0 && call.n >= kBucketedMinRows &&
+        global_in_l2) {
+      const double rows_a_group = tiled_rows(make_smem_layout(plan, skew_slots), plan) / std::max(s_heavy, 1.0);
       skew_bucketed             = nacc / std::max(1.0, std::min(rows_a_group, 16.0)) > 2.4;
     }
-    bool skew_stream = false;
+    bool skew_tiled = false;
     if (strategy == GBX_STRATEGY_AUTO) {
       // measured on B200 (100M rows, 12 accumulators): at 100 groups the shared
       // table with 32/64-bit shared atomics 4.0 ms, warp-private tables 7.2 ms;
       // at 1e4 groups the L2-resident global table 9.4 ms, the partitioned
       // path 21.4 ms; at 1e6 groups (table beyond L2) 32.6 ms against 17.2 ms
       if (est * 2.0 <= static_cast<double>(s_max)) strategy = GBX_STRATEGY_PRIVATIZED;
-      else if (stream_slots > 0) {
+      else if (skew_slots > 0) {
         strategy    = skew_bucketed ? GBX_STRATEGY_BUCKETED : GBX_STRATEGY_PRIVATIZED;
-        skew_stream = !skew_bucketed;
+        skew_tiled = !skew_bucketed;
         // the rare keys land in the global table: room for more of them than
         // the sample saw
         cap = std::min<uint64_t>(cap * 4, 1ULL << 31);
@@ -1493,13 +1494,13 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
         GBX_CUDA(launch_agg_warp(plan, t, make_smem_layout(plan, s_warp), call.n, call.dev.num_sms, max_probes, s));
       } else if (strategy == GBX_STRATEGY_PRIVATIZED) {
         uint32_t S = static_cast<uint32_t>(std::min<uint64_t>(next_pow2(static_cast<uint64_t>(std::max(2.0 * est, 64.0))), s_max));
-        if (skew_stream) S = stream_slots;
+        if (skew_tiled) S = skew_slots;
         const SmemLayout sl = make_smem_layout(plan, S);
         const int block = 512;
         int grid        = call.dev.num_sms * std::max<int>(1, std::min<int>(4, static_cast<int>((200 * 1024) / (sl.total + 1024))));
         int64_t max_grid = (call.n + block * 4 - 1) / (block * 4);
         grid             = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(grid, max_grid)));
-        if (skew_stream) {
+        if (skew_tiled) {
           // skewed keys: the tiled kernel keeps the hot keys in shared
           // memory and sends the rare keys' rows to the global table
           // a short probe: a hot key was inserted early and sits near its home
@@ -1561,9 +1562,9 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
                                1ULL << 31);
       if (strategy == GBX_STRATEGY_BUCKETED && skew_bucketed) {
         strategy    = GBX_STRATEGY_PRIVATIZED;
-        skew_stream = true;
+        skew_tiled = true;
       } else if (strategy == GBX_STRATEGY_WARP || strategy == GBX_STRATEGY_BUCKETED ||
-                 (strategy == GBX_STRATEGY_PRIVATIZED && !skew_stream)) {
+                 (strategy == GBX_STRATEGY_PRIVATIZED && !skew_tiled)) {
         strategy = GBX_STRATEGY_GLOBAL;
       }
       est = static_cast<double>(cap / 2);

@@ -128,7 +128,9 @@ __device__ __forceinline__ uint32_t valid_rows(const uint32_t* mask, int64_t i0,
 }
 
 // A 32-bit mix of a packed key for a table of the CTA's own (any mix will do
-// there; the global table's 64-bit hash costs about twice as much).
+// there; the global table's 64-bit hash costs about twice as much): the words
+// combined with odd constants, then the 32-bit finaliser of MurmurHash3
+// (Appleby, public domain).
 template <int NW>
 __device__ __forceinline__ uint32_t tile_hash(const uint64_t (&k)[NW])
 {

@@ -356,7 +356,7 @@ def test_partitioned_skewed_keys():
 @pytest.mark.parametrize("policy", [NullPolicy.EXCLUDE, NullPolicy.INCLUDE], ids=lambda p: p.name)
 def test_skewed_keys_stream_kernel(policy):
     """Zipf(1.5) keys over 50,000 ranks: AUTO keeps the hot keys in the
-    streamed-tile kernel's shared tables and sends the rare keys' rows to the
+    tiled kernel's shared tables and sends the rare keys' rows to the
     global table, so one group's partials arrive both ways (VAR shifts merged
     across them)."""
     rng = np.random.default_rng(31)
