@@ -172,28 +172,40 @@ __global__ void k_sample_distinct(const __grid_constant__ KeyPlan kp,
 }
 
 // Keys sampled at least kHeavySample times: heavy[0] += their number,
-// heavy[1] += their sampled rows; heavy[2] = the most rows of one key.
+// heavy[1] += their sampled rows; heavy[2] = the most rows of one key (set_cap
+// a multiple of 4, set_rows aligned to 16 bytes).
 __global__ void k_sample_heavy(const uint32_t* set_rows, uint64_t set_cap, unsigned long long* heavy)
 {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   uint32_t keys = 0, rows = 0, most = 0;
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < set_cap; i += stride) {
-    const uint32_t c = set_rows[i];
-    most             = max(most, c);
-    if (c >= kHeavySample) {
-      ++keys;
-      rows += c;
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < set_cap / 4; i += stride) {
+    const uint4 v       = reinterpret_cast<const uint4*>(set_rows)[i];
+    const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      most = max(most, c[j]);
+      if (c[j] >= kHeavySample) {
+        ++keys;
+        rows += c[j];
+      }
     }
   }
+  // one sum a block: the blocks' sums queue on three words
+  __shared__ uint32_t sums[3];
+  if (threadIdx.x < 3) sums[threadIdx.x] = 0;
+  __syncthreads();
   keys = __reduce_add_sync(0xffffffffu, keys);
   rows = __reduce_add_sync(0xffffffffu, rows);
   most = __reduce_max_sync(0xffffffffu, most);
-  if ((threadIdx.x & 31) != 0 || most == 0) return;
-  if (keys != 0) {
-    atomicAdd(&heavy[0], static_cast<unsigned long long>(keys));
-    atomicAdd(&heavy[1], static_cast<unsigned long long>(rows));
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sums[0], keys);
+    atomicAdd(&sums[1], rows);
+    atomicMax(&sums[2], most);
   }
-  atomicMax(&heavy[2], static_cast<unsigned long long>(most));
+  __syncthreads();
+  if (threadIdx.x < 2 && sums[threadIdx.x] != 0)
+    atomicAdd(&heavy[threadIdx.x], static_cast<unsigned long long>(sums[threadIdx.x]));
+  if (threadIdx.x == 2) atomicMax(&heavy[2], static_cast<unsigned long long>(sums[2]));
 }
 
 // Empties the sample's set, its row counts and the counters of both.
@@ -409,8 +421,8 @@ cudaError_t launch_sample(const KeyPlan& kp, int64_t n, int64_t nsample, uint64_
   int grid = grid_for(nsample, 256, num_sms * 8);
   if (kp.nwords == 1) k_sample_distinct<1><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
   else k_sample_distinct<2><<<grid, 256, 0, st>>>(kp, n, nsample, set, set_rows, set_cap - 1, counters);
-  // few warps, whose sums queue on three words
-  k_sample_heavy<<<grid_for(static_cast<int64_t>(set_cap), 256, num_sms), 256, 0, st>>>(set_rows, set_cap, heavy);
+  k_sample_heavy<<<grid_for(static_cast<int64_t>(set_cap) / 4, 256, num_sms * 2), 256, 0, st>>>(set_rows, set_cap,
+                                                                                               heavy);
   return cudaGetLastError();
 }
 
