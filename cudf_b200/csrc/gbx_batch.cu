@@ -172,7 +172,7 @@ __device__ __noinline__ void spill_rows(const Plan& plan, const BatchInst& I, in
       const int64_t r = r0 + static_cast<int64_t>(q) * step;
       uint64_t k[NW];
       src.key<NW>(r, k);
-      const int64_t g = global_slot<NW>(I.t, k, max_probes);
+      const int64_t g = global_slot<NW, false>(I.t, k, max_probes);
       if (g >= 0) accumulate_row_from<Global>(plan, src, G, g, r, I.t.status);
     }
     __syncwarp();
@@ -259,7 +259,7 @@ __device__ __forceinline__ void item_shared(const Plan& plan, const BatchInst& I
 #pragma unroll
     for (int w = 0; w < NW; ++w) k[w] = skeys[s * NW + w];
     if (srows[s] == 0) continue;
-    const int64_t g = global_slot<NW>(I.t, k, max_probes);
+    const int64_t g = global_slot<NW, false>(I.t, k, max_probes);
     if (g >= 0) merge_slot<Shared>(plan, L, s, G, g, I.t.status);
   }
 }
@@ -302,7 +302,7 @@ __device__ __forceinline__ void item_warp(const Plan& plan, const BatchInst& I, 
     const int state = warp_find_or_insert<NW>(T, plan.acc, act, k, lane, slot);
     if (__any_sync(kFull, state == ST_FOUND && slot == T.S)) special = true;
     if (state == ST_SPILL) {
-      const int64_t g = global_slot<NW>(I.t, k, max_probes);
+      const int64_t g = global_slot<NW, false>(I.t, k, max_probes);
       if (g >= 0) accumulate_row_from<Global>(plan, src, G, g, r, I.t.status);
     }
     warp_accumulate(plan, T.tb, sl, state == ST_FOUND, slot, v, lane);
@@ -322,7 +322,7 @@ __device__ __forceinline__ void item_warp(const Plan& plan, const BatchInst& I, 
     for (int w = 0; w < NW; ++w) kk[w] = keys[s * NW + w];
     const bool occupied = (s < T.S) ? !key_is_empty<NW>(kk) : special;
     if (!occupied) continue;
-    const int64_t g = global_slot<NW>(I.t, kk, max_probes);
+    const int64_t g = global_slot<NW, false>(I.t, kk, max_probes);
     if (g >= 0) merge_slot<Shared>(plan, L, s, G, g, I.t.status);
   }
 }
@@ -367,7 +367,7 @@ __device__ __forceinline__ void item_global(const Plan& plan, const BatchInst& I
     RowVals<NCH> vn;
     load_row_values(plan, src, actn, rn, vn, I.t.status);
     if (act) {
-      const int64_t g = global_slot<NW>(I.t, k, max_probes);
+      const int64_t g = global_slot<NW, false>(I.t, k, max_probes);
       if (g >= 0) accumulate_row_from<Global>(plan, LoadedRow<NCH>{&v}, G, g, r, I.t.status);
     }
     act = actn;

@@ -359,7 +359,9 @@ __device__ __forceinline__ Level<Global> global_level(const TableRef& t) { retur
 // examines max_probes slots, and where a warp waits for its lanes, so do the
 // rows beside it (20M rows of 845,000 groups in a table of 262,144: that pass
 // 38 ms one lane at a time, 88 ms by warps, 6 ms here).
-template <int NW>
+// kPoll false: without that look (the batched kernel, whose instances' tables
+// hold a few probes' groups, runs 0.7% longer with it).
+template <int NW, bool kPoll = true>
 __device__ __forceinline__ int64_t global_slot(const TableRef& t,
                                                const uint64_t (&k)[NW],
                                                uint32_t max_probes)
@@ -369,7 +371,7 @@ __device__ __forceinline__ int64_t global_slot(const TableRef& t,
     return static_cast<int64_t>(t.cap);
   }
   const int64_t s = find_or_insert<Global, NW>(reinterpret_cast<uint64_t>(t.keys), t.cap - 1, k, hash_key<NW>(k),
-                                               max_probes, t.status);
+                                               max_probes, kPoll ? t.status : nullptr);
   if (s < 0) atomicOr(t.status, S_TABLE_FULL);
   return s;
 }
