@@ -1257,19 +1257,20 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
 
     // bucket-ordered copies of the rows (radix partitioning): packed key
     // words, resolved value bits, a validity byte per row of a nullable channel
-    auto part_bufs = [&]() {
+    auto part_bufs_of = [&](Scratch& sc) {
       PartBufs pb{};
       for (int w = 0; w < plan.key.nwords; ++w)
-        pb.keys[w] = static_cast<const uint64_t*>(scratch.get(static_cast<size_t>(call.n) * 8));
+        pb.keys[w] = static_cast<const uint64_t*>(sc.get(static_cast<size_t>(call.n) * 8));
       for (int c = 0; c < plan.nchan; ++c) {
         const int width = pt_width(plan.chan[c].ptype);
         pb.col[c].width = width;
-        pb.col[c].vals  = scratch.get(static_cast<size_t>(call.n) * width);
+        pb.col[c].vals  = sc.get(static_cast<size_t>(call.n) * width);
         pb.col[c].valid =
-          plan.chan[c].a_cnt >= 0 ? static_cast<const uint8_t*>(scratch.get(static_cast<size_t>(call.n))) : nullptr;
+          plan.chan[c].a_cnt >= 0 ? static_cast<const uint8_t*>(sc.get(static_cast<size_t>(call.n))) : nullptr;
       }
       return pb;
     };
+    auto part_bufs = [&]() { return part_bufs_of(scratch); };
 
     if (strategy == GBX_STRATEGY_PARTITIONED) {
       // ---- radix-partitioned path (gbx_part.cu)
@@ -1473,6 +1474,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
     int64_t G          = 0;
     TableRef t{};
     uint32_t* map = nullptr;
+    Scratch copies(&call.alloc);  // BUCKETED: the bucket-ordered rows
     for (int attempt = 0;; ++attempt) {
       // ---- table
       t     = TableRef{};
@@ -1490,6 +1492,28 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       launches += 1;
       timer.mark(2);
       const uint32_t max_probes = static_cast<uint32_t>(std::min<uint64_t>(cap, 1u << 12));
+      PartBufs pb{}, tmp{};
+      uint32_t *rcounts = nullptr, *roffsets = nullptr, *n_kept = nullptr;
+      void* rtemp        = nullptr;
+      size_t rtemp_bytes = 0;
+      if (strategy == GBX_STRATEGY_BUCKETED) {
+        try {
+          pb       = part_bufs_of(copies);
+          tmp      = bucket_bits > 8 ? part_bufs_of(copies) : pb;  // one pass writes `pb` only
+          rcounts  = static_cast<uint32_t*>(copies.get(part_radix_count_bytes(call.n)));
+          roffsets = static_cast<uint32_t*>(copies.get(part_radix_count_bytes(call.n)));
+          GBX_CUDA(part_radix_temp_bytes(call.n, &rtemp_bytes));
+          copies.together({rtemp_bytes, sizeof(uint32_t)});
+          rtemp  = copies.get(rtemp_bytes);
+          n_kept = static_cast<uint32_t*>(copies.get(sizeof(uint32_t)));
+        } catch (const Failure& f) {
+          // no room for copies of the rows: the forms that read them in place
+          if (f.code != GBX_ERR_ALLOC) throw;
+          copies.release_all();
+          strategy   = skew_bucketed ? GBX_STRATEGY_PRIVATIZED : GBX_STRATEGY_GLOBAL;
+          skew_tiled = skew_bucketed;
+        }
+      }
       if (strategy == GBX_STRATEGY_WARP) {
         GBX_CUDA(launch_agg_warp(plan, t, make_smem_layout(plan, s_warp), call.n, call.dev.num_sms, max_probes, s));
       } else if (strategy == GBX_STRATEGY_PRIVATIZED) {
@@ -1515,15 +1539,6 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       } else if (strategy == GBX_STRATEGY_BUCKETED) {
         // radix passes into bucket order, then tiles of the bucket-ordered
         // rows grouped in shared memory (gbx_tiled.cu)
-        const PartBufs pb  = part_bufs();
-        const PartBufs tmp = bucket_bits > 8 ? part_bufs() : pb;  // one pass writes `pb` only
-        auto* rcounts      = static_cast<uint32_t*>(scratch.get(part_radix_count_bytes(call.n)));
-        auto* roffsets     = static_cast<uint32_t*>(scratch.get(part_radix_count_bytes(call.n)));
-        size_t rtemp_bytes = 0;
-        GBX_CUDA(part_radix_temp_bytes(call.n, &rtemp_bytes));
-        scratch.together({rtemp_bytes, sizeof(uint32_t)});
-        void* rtemp  = scratch.get(rtemp_bytes);
-        auto* n_kept = static_cast<uint32_t*>(scratch.get(sizeof(uint32_t)));
         GBX_CUDA(launch_part_radix_hist0(plan, call.n, bucket_bits, rcounts, nullptr, s));
         GBX_CUDA(launch_part_radix(plan, call.n, bucket_bits, n_kept, pb, tmp, rcounts, roffsets, rtemp, rtemp_bytes,
                                    d_status, /*hist0_done=*/true, s));
@@ -1551,6 +1566,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       if (cap >= (1ULL << 31) || attempt >= 3) fail(GBX_ERR_DEVICE, "hash table overflow at capacity %llu", (unsigned long long)cap);
       gb->stats.retries++;
       scratch.release_all();
+      copies.release_all();
       ctl = static_cast<unsigned long long*>(scratch.get(kCtlWords * 8));
       GBX_CUDA(cudaMemsetAsync(ctl, 0, kCtlWords * 8, s));
       d_status       = reinterpret_cast<int32_t*>(ctl + 26);
@@ -1576,7 +1592,7 @@ int gbx_groupby_aggregate(gbx_groupby* gb,
       gb->stats.bucket_slots   = static_cast<int32_t>(bucket_slots);
     }
     gb->stats.num_groups      = G;
-    gb->stats.scratch_bytes   = static_cast<int64_t>(scratch.total());
+    gb->stats.scratch_bytes   = static_cast<int64_t>(scratch.total() + copies.total());
     gb->stats.kernel_launches = launches + (G > 0 ? 1 : 0);  // + finalize
     res->num_groups           = G;
 

@@ -10,7 +10,7 @@ from cudf_b200 import Column, GroupBy, GroupByRequest, Table
 from cudf_b200 import _lib
 from cudf_b200 import aggregation as agg
 from cudf_b200 import join as J
-from cudf_b200._abi import Status
+from cudf_b200._abi import Status, Strategy
 from cudf_b200.groupby import TorchAllocator
 from oracle.oracle import HostCol
 from tests import gbx_testing as T
@@ -127,3 +127,29 @@ def test_a_join_in_a_pool_of_a_few_buffers(room):
         assert e.status == Status.ERR_ALLOC and room < 100 << 10
     else:
         assert _pairs(got) == [(i, i) for i in range(1000)]
+
+
+@pytest.mark.parametrize("columns,groups,hot", [(1, 20_000, 0.0), (5, 12_000, 0.1), (5, 1000, 0.0)],
+                         ids=["bucketed", "one_run_an_sm", "skewed"])
+def test_bucketed_calls_where_the_copies_have_no_room(columns, groups, hot):
+    """4.2M rows: copies of 33 MB a column, against a pool that gives 8 MB at a time."""
+    rng = np.random.default_rng(groups)
+    n = 4_200_000
+    k = rng.integers(0, groups, n)
+    k[rng.random(n) < hot] = 3
+    vals = [rng.integers(-50, 50, n).astype(np.float64) for _ in range(columns)]
+    valid = [rng.random(n) >= 0.1 for _ in vals]
+    gb = GroupBy(Table([T.device_column(HostCol(k.astype(np.int64)))]))
+    reqs = [GroupByRequest(T.device_column(HostCol(v, ok)), [agg.sum(), agg.count(), agg.mean()])
+            for v, ok in zip(vals, valid)]
+    free = gb.aggregate(reqs)
+    assert gb.last_stats()["strategy"] == Strategy.BUCKETED
+    tight = gb.aggregate(reqs, allocator=TightAllocator(8 << 20))
+    assert gb.last_stats()["strategy"] != Strategy.BUCKETED
+    for gk, res in (free, tight):
+        key = gk.columns()[0].to_numpy()[0]
+        assert np.array_equal(np.sort(key), np.unique(k))
+        for v, ok, t in zip(vals, valid, res):
+            want = np.bincount(k[ok], weights=v[ok], minlength=groups)  # whole numbers: exact in any order
+            assert np.array_equal(t.columns()[0].to_numpy()[0], want[key])
+            assert np.array_equal(t.columns()[1].to_numpy()[0], np.bincount(k[ok], minlength=groups)[key])
