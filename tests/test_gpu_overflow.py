@@ -35,3 +35,16 @@ def test_overflowing_table(strategy, two_words):
     got, want = T.assert_parity(keys, [(HostCol(v), AGGS)], strategy=strategy)
     assert got["stats"]["retries"] >= 1
     assert got["num_groups"] == want["num_groups"]
+
+
+def test_overflow_of_a_wide_skewed_plan():
+    """Bucketed for the 300 keys the sample sees; the other 20,000 overflow its table, and the skewed form, which
+    spills them to a larger global table, takes over."""
+    n, m = 4_300_000, 1 << 16
+    rng = np.random.default_rng(5)
+    k = rng.integers(0, 20_000, n)
+    k[((np.arange(m) + 0.5) * n / m).astype(np.int64)] = np.arange(m) % 300
+    cols = [HostCol(rng.integers(-50, 50, n).astype(np.float64), rng.random(n) >= 0.1) for _ in range(3)]
+    aggs = [(Kind.SUM, 0), (Kind.MIN, 0), (Kind.MAX, 0), (Kind.VARIANCE, 1)]
+    got, _ = T.assert_parity([HostCol(k.astype(np.int64))], [(c, aggs) for c in cols])
+    assert got["stats"]["retries"] == 1 and got["stats"]["strategy"] == Strategy.PRIVATIZED
